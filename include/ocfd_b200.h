@@ -115,8 +115,8 @@ int ocfd_b200_uniform_metrics(const ocfd_b200_ctx *ctx);
  * 5: the walk with every face through one in-loop dispatch (the path of the
  * schemes other than UP7, WENO7 and the hybrid scheme in variant 4 too);
  * 6: the in-line walk alone (characteristic hybrid scheme and WENO7 only);
- * 7: as 4 with every UP7 walk through the shared-memory ring; 8: as 4 with
- * the y and z marches in FP64 as well (as fast as the ring there).  All
+ * 7: as 4 with the y and z UP7 walks through the shared-memory ring; 8: as 4
+ * (it once chose the marches in FP64, which 4 now takes too).  All
  * agree to the parity bound (WENO weights amplify the different multiply-add
  * contractions); 4, 7 and 8 agree bit for bit.  Other values: OCFD_ERR_ARG. */
 int ocfd_b200_set_sweep_impl(ocfd_b200_ctx *ctx, int impl);

@@ -22,11 +22,10 @@ namespace ocfd {
 cudaError_t launch_sensor(const Params &p, cudaStream_t st);
 cudaError_t launch_q_criterion(const Params &p, double *q, cudaStream_t st);
 cudaError_t launch_time_average(const Params &p, double *mean5, int n, cudaStream_t st);
-bool march_tensor_map(const Params &p, const void *base, int elem_bytes, int dir, CUtensorMap *out);
 bool march_supported(const Params &p, int dir);
 cudaError_t march_prepare();
 cudaError_t vdiv_prepare();
-cudaError_t launch_march_dir(const Params &p, const CUtensorMap &tm, int dir, cudaStream_t st);
+cudaError_t launch_march_dir(const Params &p, int dir, cudaStream_t st);
 cudaError_t launch_ghost(const Params &p, double *const *fields, const int *dirmask, int nf, cudaStream_t st);
 cudaError_t launch_ghost32(const Params &p, float *const *fields, const int *dirmask, int nf, cudaStream_t st);
 cudaError_t launch_prims_to_fp32(const Params &p, cudaStream_t st);
@@ -143,15 +142,9 @@ struct ocfd_b200_ctx {
     float sw_conf_logit = 0.0f;
     int walk4[3] = {1, 1, 1};
     double walk4_threshold = 0.002;     // deferred cells per cell above which the inline walk is used
-    // the UP7 walk of the y and z sweeps as per-lane marches over staged
-    // pencil tiles (ocfd_march.cu): tensor maps of the FP64 and FP32
-    // primitives per direction (y, z).  march: 0 the shared-memory ring walk
-    // everywhere (sweep variant 7), 1 the march in the precision form only
-    // (default: in FP64 the ring walk measured as fast), 2 the march in both
-    // forms (variant 8)
-    CUtensorMap tm64[2];
-    CUtensorMap tm32[2];
-    bool tm64_ok = false, tm32_ok = false;
+    // the UP7 walk of the y and z sweeps as per-lane marches (ocfd_march.cu);
+    // 0: the shared-memory ring walk there too (sweep variant 7)
+    bool march_ok = false;      // the marches' shared-memory sizes are set
     bool vdiv_ok = true;        // the staged divergence kernel can be launched
     // running time averages of d, u, v, w, T (5 interior fields, allocated on
     // first use) and the number of samples in them
@@ -384,9 +377,7 @@ extern "C" int ocfd_b200_create(const ocfd_b200_config *cfg, ocfd_b200_ctx **out
     }
     // the staged divergence kernel is used only when its shared-memory size is set
     if (ocfd::vdiv_prepare() != cudaSuccess) { cudaGetLastError(); p.vis_impl = 1; ctx->vdiv_ok = false; }
-    ctx->tm64_ok = ocfd::march_prepare() == cudaSuccess &&
-                   ocfd::march_tensor_map(p, ctx->prim_buf, 8, 1, &ctx->tm64[0]) &&
-                   ocfd::march_tensor_map(p, ctx->prim_buf, 8, 2, &ctx->tm64[1]);
+    ctx->march_ok = ocfd::march_prepare() == cudaSuccess;
     cudaGetLastError();
 
     if ((e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking)) != cudaSuccess ||
@@ -645,10 +636,8 @@ static int sweeps_auto(ocfd_b200_ctx *ctx) {
         if (w[d]) {
             CK(ocfd::launch_sweep4_dir(p, d, ctx->stream), "inviscid sweeps");
             ctx->launches += 1;
-        } else if (d > 0 && ctx->march > (p.mixed ? 0 : 1) && ocfd::march_supported(p, d) &&
-                   (p.mixed ? ctx->tm32_ok : ctx->tm64_ok)) {
-            CK(ocfd::launch_march_dir(p, p.mixed ? ctx->tm32[d - 1] : ctx->tm64[d - 1], d, ctx->stream),
-               "inviscid sweeps");
+        } else if (d > 0 && ctx->march && ctx->march_ok && ocfd::march_supported(p, d)) {
+            CK(ocfd::launch_march_dir(p, d, ctx->stream), "inviscid sweeps");
             ctx->launches += 2;
         } else {
             CK(ocfd::launch_sweep3_dir(p, d, ctx->stream), "inviscid sweeps");
@@ -928,8 +917,6 @@ extern "C" int ocfd_b200_set_precision(ocfd_b200_ctx *ctx, int form) {
     p.ev32 = ctx->prec_buf + 5 * (size_t)p.lapN;
     p.pfil32 = ctx->prec_buf + 17 * (size_t)p.lapN;
     p.du32 = ctx->prec_buf + 18 * (size_t)p.lapN;
-    ctx->tm32_ok = ocfd::march_tensor_map(p, ctx->prec_buf, 4, 1, &ctx->tm32[0]) &&
-                   ocfd::march_tensor_map(p, ctx->prec_buf, 4, 2, &ctx->tm32[1]);
     p.mixed = 1;
     if (ctx->have_state) {
         CK(ocfd::launch_prims_to_fp32(p, ctx->stream), "FP32 primitives");
@@ -1140,7 +1127,7 @@ extern "C" int ocfd_b200_set_walk_threshold(ocfd_b200_ctx *ctx, double frac) {
 
 extern "C" int ocfd_b200_set_sweep_impl(ocfd_b200_ctx *ctx, int impl) {
     if (!ctx || impl < 4 || impl > 8) return OCFD_ERR_ARG;
-    ctx->march = impl == 7 ? 0 : (impl == 8 ? 2 : 1);
+    ctx->march = impl == 7 ? 0 : 1;
     ctx->p.sweep_impl = impl >= 7 ? 4 : impl;
     return OCFD_OK;
 }

@@ -1,21 +1,28 @@
 // ocfd_march.cu -- the UP7 walk of the y and z sweeps as per-lane marches
-// over TMA-staged pencil tiles (sm_100a; FP64, and FP32 for the precision form).
+// (sm_100a; FP64, and FP32 for the precision form), and the tensor-map encoder.
 //
 // Same results as the UP7 walk of ocfd_sweep3.cu (the reference's
 // OCFD_d{y,z}1/2 chain with the hybrid scheme's UP7 faces, src/OCFD_Schemes.cu:159-381,
-// 865-907): every split point and face flux formed once, du in the
-// reference's y+, y- (z+, z-) order, one writer per element.
+// 865-907): every point split once, every face's flux formed once, one
+// writer per du element.
 //
 // Organisation.  A warp owns 32 consecutive x columns of one z (y sweep) or
-// y (z sweep) and a segment of the line; each lane walks its own column.
-// The primitives of the pencil (32 columns x 8 points x 5 fields) arrive in
-// shared memory by one 4-D bulk tensor copy per chunk, double-buffered per
-// warp behind an mbarrier, so the loads of the next chunk run while the
-// lane computes.  The lane keeps the split values of the last 8 points in
-// registers (the window of the face it forms next); the 8-point chunk is
-// unrolled, so a point's window slot is a compile-time index and nothing is
-// shifted.  No shared-memory window reads remain (the ring walk reads 70
-// per face), and no block barrier is taken.
+// y (z sweep) and a segment of the line; each lane walks its own column.  UP7
+// is linear, so the lane keeps no window of split values: it keeps the
+// running sums of the eight faces that the newest point still reaches
+// (5 fields each, both signs in one sum), adds the point's split values to
+// all of them and takes the finished one.  The 8-point body is unrolled, so a
+// face's slot is a compile-time index.  That is 40 values of state where the
+// window took 75, and 15 multiply-adds a field and cell where the two
+// quotients of each face took 34 operations.
+// Primitives, the cell's du and (curvilinear grids) the metrics are copied
+// to the lane's own shared-memory slots by cp.async STAGES - 1 points ahead; a
+// lane reads only what it copied, so the walk takes no barrier at all.
+// Bounds: FP64 by memory latency and bandwidth (120 B a cell and direction,
+// 53 % of DRAM peak with 12 warps an SM), FP32 by instruction issue (68 %).
+// At 160^3, y / z: FP64 110 / 108 us against 158 / 171 for the ring walk; FP32
+// 78 / 79 us against 112 / 107 for a march over tiles from the tensor copy
+// engine with a register window of split values.
 //
 // Faces that are not plain UP7 (hybrid flags other than 1, faces within
 // reach of a boundary closure) defer the cells on both sides, and the first
@@ -38,30 +45,36 @@ namespace {
 using namespace walk;
 
 constexpr int MW = 4;          // warps per block
-constexpr int CH = 8;          // points per staged chunk (the window length)
-using namespace tma;
+constexpr int STAGES = 4;      // points in flight or in use per lane
 
-template <typename R>
-constexpr int chunk_elems() { return 5 * CH * 32; }     // [field][point][column]
+__device__ __forceinline__ void copy_async(double *dst, const double *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(tma::smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async(float *dst, const float *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(tma::smem_u32(dst)), "l"(src) : "memory");
+}
 
-// DIR: 1 (y) or 2 (z).  tm: the primitives the stencils read as a 4-D
-// tensor [x: row pitch][y: LAP rows][z: LAP planes][field: 5], box
-// 32 x CH x 1 x 5 (y) or 32 x 1 x CH x 5 (z).
+// values staged per point: 5 primitives and 5 du, and on a curvilinear grid
+// the point's metric row and the cell's Jacobian (FP64 in both forms)
+template <bool UNI, typename R>
+struct Stage {
+    R q[10][32 * MW];
+    double met[UNI ? 1 : 4][UNI ? 1 : 32 * MW];
+};
+
+// blocks per SM the register budget is fitted to
+template <typename R> constexpr int march_blocks() { return sizeof(R) == 8 ? 3 : 5; }
+
 template <int DIR, bool UNI, bool EPS0, typename R>
-__global__ void __launch_bounds__(32 * MW, sizeof(R) == 8 ? 2 : 3)
-k_march(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm, int seg_len) {
+__global__ void __launch_bounds__(32 * MW, march_blocks<R>()) k_march(const __grid_constant__ Params p, int seg_len) {
     static_assert(DIR == 1 || DIR == 2, "the march covers the y and z sweeps");
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ unsigned long long bars[MW][2];
-    constexpr int CE = chunk_elems<R>();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    Stage<UNI, R> *stage = reinterpret_cast<Stage<UNI, R> *>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31;
     const int ngx = (p.nx + 31) / 32;
     const int n3 = DIR == 1 ? p.nz : p.ny;
-    const long long grp = (long long)blockIdx.x * MW + wid;
+    const long long grp = (long long)blockIdx.x * MW + (tid >> 5);
     if (grp >= (long long)ngx * n3) return;                   // the whole warp
-    R *buf = reinterpret_cast<R *>(smem_raw) + (size_t)wid * 2 * CE;
-    unsigned long long *bar = bars[wid];
-
     const int g = (int)(grp % ngx), c3 = (int)(grp / ngx);
     const int x = g * 32 + lane;
     const bool colok = x < p.nx;
@@ -85,132 +98,98 @@ k_march(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm
     R *__restrict__ du = du_r<R>(p);
     const long long N = p.N;
     const bool hybrid = p.scheme_invis == 310;
-    const R h = (R)(DIR == 1 ? p.hy : p.hz), ih = (R)p.inv_h[DIR];
+    const R sc0 = UNI ? up7_scale((R)p.mc[M_AJAC], p.inv_h[DIR]) : (R)0.0;
 
-    // points P0 .. y1+3 in chunks of CH; point P sits in window slot (P - P0) % CH
-    const int P0 = y0 - 4;
-    const int nch = (y1 - y0 + 8 + CH - 1) / CH;
-    if (lane == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        fence_mbar_init();
-    }
-    __syncwarp();
-    auto issue = [&](int c) {           // lane 0: chunk c into buffer c % 2
-        const int b = c & 1;
-        mbar_expect_tx(&bar[b], (unsigned)(CE * sizeof(R)));
-        const int cx = OCFD_LAP + g * 32, cp = OCFD_LAP + P0 + c * CH, cq = OCFD_LAP + c3;
-        if (DIR == 1) load_4d(buf + b * CE, &tm, cx, cp, cq, 0, &bar[b]);
-        else          load_4d(buf + b * CE, &tm, cx, cq, cp, 0, &bar[b]);
-    };
-    if (lane == 0) {
-        issue(0);
-        if (nch > 1) issue(1);
-    }
-
-    // flag of face F+1/2 is entry F+1: chunk c, slot t holds face F = P - 4,
-    // entry P0 + c*CH + t - 3, used when y0 <= entry <= y1
-    auto load_flags = [&](int c, int (&hf)[CH]) {
+    // points P0 .. y1+3; point P is staged in slot (P - P0) % STAGES.  The
+    // offsets run along with the walk (formed from P, the unrolled body's
+    // eight of each would all stay in registers).
+    const int P0 = y0 - 4, P1 = y1 + 3;
+    long long of = base + (long long)P0 * sd;                 // LAP offset of the next point to fetch
+    long long cf = cb + (long long)(y0 - 4 - 4) * cst;        // and the cell it completes
+    long long cs = cf;                                        // the cell that the current point completes
+    const int8_t *fp_ = fl + (long long)(y0 - 7) * fst;       // flag of the face that the next point completes
+    auto fetch = [&](int P, int s) {
+        if (P <= P1) {
+            Stage<UNI, R> &S = stage[s];
+            const long long o = OCFD_IDX(p, of, p.lapN);
 #pragma unroll
-        for (int t = 0; t < CH; t++) {
-            const int e = P0 + c * CH + t - 3;
-            hf[t] = (hybrid && colok && e >= y0 && e <= y1) ? flag_at(p, DIR, fl, (long long)e * fst) : 2;
-        }
-    };
-    // the chunk's flags, one byte each (flags are small integers)
-    auto pack = [](const int (&hf)[CH]) {
-        unsigned long long v = 0;
+            for (int m = 0; m < 5; m++) copy_async(&S.q[m][tid], prim_r<R>(p, m) + o);
+            if constexpr (!UNI) {
 #pragma unroll
-        for (int t = 0; t < CH; t++) v |= (unsigned long long)(hf[t] & 0xff) << (8 * t);
-        return v;
-    };
-    int hn[CH];
-    load_flags(0, hn);
-    unsigned long long hpk = pack(hn);
-
-    R wp[CH][5], wm[CH][5];             // split values of the window's points
-    R prv[10];
-#pragma unroll
-    for (int m = 0; m < 10; m++) prv[m] = (R)0.0;
-#pragma unroll
-    for (int t = 0; t < CH; t++)
-#pragma unroll
-        for (int m = 0; m < 5; m++) { wp[t][m] = (R)0.0; wm[t][m] = (R)0.0; }
-    int prv_slow = 0;
-    unsigned phase = 0;                 // bit b: parity of buffer b's next phase
-
-    for (int c = 0; c < nch; c++) {
-        const int b = c & 1;
-        if (c + 1 < nch) load_flags(c + 1, hn);
-        {
-            long long it = 0;
-            while (!mbar_try_wait(&bar[b], (phase >> b) & 1u)) {
-                if (++it > WAIT_LIMIT) {
-                    if (lane == 0) atomicExch(p.kerr, 1);
-                    // the other buffer's copy, if one is in flight, lands
-                    // before the block's shared memory goes away
-                    if (c + 1 < nch) {
-                        long long it2 = 0;
-                        while (!mbar_try_wait(&bar[b ^ 1], (phase >> (b ^ 1)) & 1u) && ++it2 <= WAIT_LIMIT) {}
-                    }
-                    return;
-                }
+                for (int m = 0; m < 3; m++) copy_async(&S.met[m][tid], p.met[M_AKX + 3 * DIR + m] + o);
             }
-            phase ^= 1u << b;
+            if (P - 4 >= y0) {
+                const long long ci = OCFD_IDX(p, cf, N);
+#pragma unroll
+                for (int m = 0; m < 5; m++) copy_async(&S.q[5 + m][tid], du + m * N + ci);
+                if constexpr (!UNI) copy_async(&S.met[3][tid], p.met[M_AJAC] + OCFD_IDX(p, of - 4 * sd, p.lapN));
+            }
         }
-        const R *cbuf = buf + b * CE;
+        of += sd;
+        cf += cst;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // flag of face F+1/2, F = P - 4, is entry F+1 = P - 3
+    auto next_flag = [&](int P) {
+        const int e = P - 3;
+        const int8_t *f = fp_;
+        fp_ += fst;
+        return (hybrid && e >= y0 && e <= y1) ? flag_at(p, DIR, f, 0) : 2;
+    };
 #pragma unroll
-        for (int t = 0; t < CH; t++) {
-            const int P = P0 + c * CH + t;
-            if (P <= y1 + 3) {
+    for (int s = 0; s < STAGES - 1; s++) fetch(P0 + s, s);
+    int hf[4];                           // flags of points P .. P+2, loaded three points ahead
+#pragma unroll
+    for (int s = 0; s < 3; s++) hf[s] = next_flag(P0 + s);
+    hf[3] = 2;
+
+    R S[8][5];                           // face F's sum in slot (F - P0 + 4) % 8
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int m = 0; m < 5; m++) S[j][m] = (R)0.0;
+    int prv_slow = 0;
+
+    for (int Pc = P0; Pc <= P1; Pc += 8) {
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+            const int P = Pc + t;
+            if (P <= P1) {
+                fetch(P + STAGES - 1, (t + STAGES - 1) % STAGES);
+                hf[(t + 3) & 3] = next_flag(P + 3);
+                asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+                const Stage<UNI, R> &G = stage[t % STAGES];
+                R q[5], fp[5], fm[5];
+#pragma unroll
+                for (int m = 0; m < 5; m++) q[m] = G.q[m][tid];
+                if constexpr (UNI) {
+                    split_point<DIR, UNI, EPS0>(p, 0, q[0], q[1], q[2], q[3], q[4], fp, fm);
+                } else {
+                    const R cc = div_const(sqrt_r(q[4]), (R)p.Ama, (R)p.inv_Ama);
+                    sw_split(q[0] * (R)p.tmp0, q[1], q[2], q[3], cc, (R)G.met[0][tid], (R)G.met[1][tid],
+                             (R)G.met[2][tid], (R)p.Gamma, (R)p.epsl_sw, (R)p.split_C1, (R)p.split_C3, fp, fm);
+                }
+                // stencil entry k of face F = P - 4 + j is point P for k = 7 - j
                 const int F = P - 4;
-                // du of the next step's cell into L1 now, so that its read
-                // after this step's faces does not wait on DRAM
-                if (colok && F + 1 >= y0 && F + 1 < y1) {
-                    const R *q = du + cb + (long long)(F + 1) * cst;
-#pragma unroll
-                    for (int m = 0; m < 5; m++) prefetch_l1(q + m * N);
-                }
-                // this step's cell: its du is read before the faces are formed
-                R old[5];
-                if (colok && F >= y0) {
-#pragma unroll
-                    for (int m = 0; m < 5; m++) old[m] = du[m * N + cb + (long long)F * cst];
-                }
-                // + sign of face F+1/2: points F-3 .. F+3 (slots t+1 .. t+7)
-                R cur[10];
+                R diff[5];
 #pragma unroll
                 for (int m = 0; m < 5; m++) {
-                    R v[8];
+                    S[t][m] = fma_r(up7_c<R>(0), fm[m], S[t][m]);            // face F is complete
+                    diff[m] = S[t][m] - S[(t + 7) & 7][m];
+                    S[(t + 7) & 7][m] = up7_c<R>(0) * fp[m];                  // face F + 7 begins
 #pragma unroll
-                    for (int k = 0; k < 7; k++) v[k] = wp[(t + 1 + k) & (CH - 1)][m];
-                    v[7] = (R)0.0;
-                    cur[m] = up7_p_q(v);
-                }
-                // the split of point P into slot t (whose point P-8 is done)
-                {
-                    R q[5];
-#pragma unroll
-                    for (int m = 0; m < 5; m++) q[m] = cbuf[(m * CH + t) * 32 + lane];
-                    split_point<DIR, UNI, EPS0>(p, base + (long long)P * sd, q[0], q[1], q[2], q[3], q[4],
-                                                wp[t], wm[t]);
+                    for (int j = 1; j < 7; j++) {
+                        R &s = S[(t + j) & 7][m];
+                        s = fma_r(up7_c<R>(7 - j), fp[m], s);
+                        s = fma_r(up7_c<R>(j), fm[m], s);
+                    }
                 }
                 if (F >= y0 - 1) {
-                    // - sign of face F+1/2: points F-2 .. F+4 (slots t+2 .. t+8)
-#pragma unroll
-                    for (int m = 0; m < 5; m++) {
-                        R v[8];
-                        v[0] = (R)0.0;
-#pragma unroll
-                        for (int k = 1; k < 8; k++) v[k] = wm[(t + 1 + k) & (CH - 1)][m];
-                        cur[5 + m] = up7_m_q(v);
-                    }
-                    const int hflag = (int)(signed char)((hpk >> (8 * t)) & 0xff);
-                    const int slow = !up7_face(p, hflag) || near_closure(p, DIR, F, n);
-                    if (F >= y0) {               // cell F: faces F-1/2 (prv) and F+1/2 (cur)
+                    const int slow = !up7_face(p, hf[t & 3]) || near_closure(p, DIR, F, n);
+                    if (F >= y0) {               // cell F: faces F-1/2 and F+1/2
                         bool defer = colok && (slow || prv_slow);
                         if (p.has_bnd) defer = defer || (colok && rule_cell(p, DIR, F, n));
-                        const long long ci = OCFD_IDX(p, cb + (long long)F * cst, N);
+                        const long long ci = OCFD_IDX(p, cs, N);
                         const unsigned mask = __ballot_sync(FULL, defer);
                         if (mask) {              // one atomic per warp
                             const int leader = __ffs(mask) - 1;
@@ -220,60 +199,53 @@ k_march(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm
                             if (defer) p.defer[DIR][OCFD_IDX(p, (long long)slot + __popc(mask & ((1u << lane) - 1u)), p.N)] = (unsigned)ci;
                         }
                         if (colok && !defer) {
-                            const R aj = (R)metric<UNI>(p, M_AJAC, base + (long long)F * sd);
-                            add_du<false>(du, N, ci, aj, h, ih, cur, prv, old);
+                            const R sc = UNI ? sc0 : up7_scale((R)G.met[UNI ? 0 : 3][UNI ? 0 : tid], p.inv_h[DIR]);
+#pragma unroll
+                            for (int m = 0; m < 5; m++) du[m * N + ci] = fma_r(sc, diff[m], G.q[5 + m][tid]);
                         }
                     }
-#pragma unroll
-                    for (int m = 0; m < 10; m++) prv[m] = cur[m];
                     prv_slow = slow;
                 }
+                cs += cst;
             }
         }
-        __syncwarp();                    // every lane is done with buffer b
-        if (lane == 0 && c + 2 < nch) issue(c + 2);
-        if (c + 1 < nch) hpk = pack(hn);
     }
 }
 
 // ---------------------------------------------------------------------------
-// host side: tensor maps and launches
+// host side
 // ---------------------------------------------------------------------------
-
-template <typename R>
-constexpr size_t smem_bytes() { return (size_t)MW * 2 * chunk_elems<R>() * sizeof(R); }
 
 template <int DIR, bool UNI, bool EPS0, typename R>
 cudaError_t set_smem() {
     return cudaFuncSetAttribute(k_march<DIR, UNI, EPS0, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem_bytes<R>());
+                                (int)(STAGES * sizeof(Stage<UNI, R>)));
 }
 
 template <int DIR, bool UNI, bool EPS0, typename R>
-cudaError_t launch_one(const Params &p, const CUtensorMap &tm, cudaStream_t st) {
-    const int ngx = (p.nx + 31) / 32;
+cudaError_t launch_one(const Params &p, cudaStream_t st) {
     const int n3 = DIR == 1 ? p.nz : p.ny;
     const int n = DIR == 1 ? p.ny : p.nz;
-    const long long groups = (long long)ngx * n3;
-    // segments of a line, so that there are about three waves of warps; a
-    // segment re-splits 7 points
-    constexpr int BLOCKS_PER_SM = sizeof(R) == 8 ? 2 : 3;
-    const long long want = 3LL * 148 * BLOCKS_PER_SM * MW;
-    long long nseg = (want + groups - 1) / groups;
-    const long long maxseg = n / 32 > 0 ? n / 32 : 1;
-    if (nseg > maxseg) nseg = maxseg;
-    if (nseg < 1) nseg = 1;
-    int seg_len = (int)((n + nseg - 1) / nseg);
-    nseg = (n + seg_len - 1) / seg_len;
-    const size_t smem = smem_bytes<R>();
-    dim3 grid((unsigned)((groups + MW - 1) / MW), (unsigned)nseg);
-    k_march<DIR, UNI, EPS0, R><<<grid, 32 * MW, smem, st>>>(p, tm, seg_len);
+    const long long blocks = ((long long)((p.nx + 31) / 32) * n3 + MW - 1) / MW;
+    // segments of a line: a segment walks 8 points more than its cells, so
+    // the split with the fewest points on the busiest SM slot
+    const long long slots = 148LL * march_blocks<R>();
+    int seg_len = n;
+    long long best = -1;
+    for (int nseg = 1; nseg <= (n + 7) / 8; nseg++) {
+        const int len = (n + nseg - 1) / nseg;
+        const long long rounds = (blocks * ((n + len - 1) / len) + slots - 1) / slots;
+        const long long cost = rounds * (len + 8 + 4);
+        if (best < 0 || cost < best) { best = cost; seg_len = len; }
+    }
+    const dim3 grid((unsigned)blocks, (unsigned)((n + seg_len - 1) / seg_len));
+    k_march<DIR, UNI, EPS0, R><<<grid, 32 * MW, STAGES * sizeof(Stage<UNI, R>), st>>>(p, seg_len);
     return cudaGetLastError();
 }
 
 template <bool UNI, bool EPS0, typename R>
-cudaError_t launch_dir_t(const Params &p, const CUtensorMap &tm, int dir, cudaStream_t st) {
-    return dir == 1 ? launch_one<1, UNI, EPS0, R>(p, tm, st) : launch_one<2, UNI, EPS0, R>(p, tm, st);
+cudaError_t launch_dir_t(const Params &p, int dir, cudaStream_t st) {
+    return dir == 1 ? launch_one<1, UNI, EPS0, R>(p, st) : launch_one<2, UNI, EPS0, R>(p, st);
 }
 
 }  // namespace
@@ -324,40 +296,27 @@ bool encode_map_4d(const void *base, int elem_bytes, const unsigned long long di
     return r == CUDA_SUCCESS;
 }
 
-// A 4-D tensor map over five LAP-box fields that start at base, field
-// stride lapN elements: dims [pitch, ny + 2 LAP, nz + 2 LAP, 5], box
-// 32 x CH x 1 x 5 along y (dir 1) or 32 x 1 x CH x 5 along z (dir 2).
-bool march_tensor_map(const Params &p, const void *base, int elem_bytes, int dir, CUtensorMap *out) {
-    if (dir != 1 && dir != 2) return false;
-    const unsigned long long eb = (unsigned long long)elem_bytes;
-    const unsigned long long dims[4] = { (unsigned long long)p.ys, (unsigned long long)(p.ny + 2 * OCFD_LAP),
-                                         (unsigned long long)(p.nz + 2 * OCFD_LAP), 5 };
-    const unsigned long long strides[3] = { p.ys * eb, p.zs * eb, p.lapN * eb };
-    const unsigned box[4] = { 32, dir == 1 ? (unsigned)CH : 1u, dir == 2 ? (unsigned)CH : 1u, 5 };
-    return encode_map_4d(base, elem_bytes, dims, strides, box, out);
-}
-
 // The march covers the UP7 walk's schemes (the hybrid scheme, UP7 without
 // projection) on the y and z sweeps.
 bool march_supported(const Params &p, int dir) {
     const bool fast_scheme = (p.scheme_invis == 301 && !p.charteric) || p.scheme_invis == 310;
-    return (dir == 1 || dir == 2) && fast_scheme && p.defer[0] != nullptr && p.kerr != nullptr;
+    return (dir == 1 || dir == 2) && fast_scheme && p.defer[0] != nullptr;
 }
 
 // one direction: the march, then the fix-up of its deferred cells (the
 // caller clears the deferred counters once per stage, as for the ring walk)
-cudaError_t launch_march_dir(const Params &p, const CUtensorMap &tm, int dir, cudaStream_t st) {
+cudaError_t launch_march_dir(const Params &p, int dir, cudaStream_t st) {
     cudaError_t e;
     if (p.mixed) {
-        e = p.uniform_metrics ? (p.epsl_sw == 0.0 ? launch_dir_t<true, true, float>(p, tm, dir, st)
-                                                  : launch_dir_t<true, false, float>(p, tm, dir, st))
-                              : launch_dir_t<false, false, float>(p, tm, dir, st);
+        e = p.uniform_metrics ? (p.epsl_sw == 0.0 ? launch_dir_t<true, true, float>(p, dir, st)
+                                                  : launch_dir_t<true, false, float>(p, dir, st))
+                              : launch_dir_t<false, false, float>(p, dir, st);
         if (e != cudaSuccess) return e;
         return launch_sweep4_fix(p, dir, st);
     }
-    e = p.uniform_metrics ? (p.epsl_sw == 0.0 ? launch_dir_t<true, true, double>(p, tm, dir, st)
-                                              : launch_dir_t<true, false, double>(p, tm, dir, st))
-                          : launch_dir_t<false, false, double>(p, tm, dir, st);
+    e = p.uniform_metrics ? (p.epsl_sw == 0.0 ? launch_dir_t<true, true, double>(p, dir, st)
+                                              : launch_dir_t<true, false, double>(p, dir, st))
+                          : launch_dir_t<false, false, double>(p, dir, st);
     if (e != cudaSuccess) return e;
     return launch_sweep3_fix(p, dir, st);
 }

@@ -103,22 +103,24 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep3(const __grid_constant_
         }
     }
     __syncwarp();
-    R carry[10], cur[10];
+    // FAST: the face's sum of both signs (face_up7_sum); else both signs
+    constexpr int NV = FAST ? 5 : 10;
+    R carry[NV], cur[NV];
 #pragma unroll
-    for (int m = 0; m < 10; m++) cur[m] = (R)0.0;
+    for (int m = 0; m < NV; m++) cur[m] = (R)0.0;
     int slow = 0, carry_slow = 0;
     if (ly == 0 && colok) {
         const int hf = hybrid ? flag_at(p, DIR, fl, (long long)y0 * fst) : 2;
         if constexpr (FAST) {
             slow = !up7_face(p, hf) || near_closure(p, DIR, y0 - 1, n);
-            if (!slow) face_up7<RING, LC>(ring, col, y0 - 1, cur);
+            if (!slow) face_up7_sum<RING, LC>(ring, col, y0 - 1, cur);
         } else {
-            if constexpr (sizeof(R) == 8)
+            if constexpr (sizeof(R) == 8 && !FAST)
                 face_flux<RING, LC, UNI>(p, DIR, ring, col, y0 - 1, n, hf, base + (long long)(y0 - 1) * sd, sd, cur);
         }
     }
 #pragma unroll
-    for (int m = 0; m < 10; m++) carry[m] = __shfl_sync(FULL, cur[m], col);
+    for (int m = 0; m < NV; m++) carry[m] = __shfl_sync(FULL, cur[m], col);
     if constexpr (FAST) carry_slow = __shfl_sync(FULL, slow, col);
 
     // the primitives of this lane's next point and the flag of its next
@@ -146,14 +148,14 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep3(const __grid_constant_
         }
         if constexpr (FAST) {
             slow = valid && (!up7_face(p, hflag) || near_closure(p, DIR, F, n));
-            if (valid && !slow) face_up7<RING, LC>(ring, col, F, cur);
+            if (valid && !slow) face_up7_sum<RING, LC>(ring, col, F, cur);
         } else {
             if constexpr (sizeof(R) == 8)
                 if (valid) face_flux<RING, LC, UNI>(p, DIR, ring, col, F, n, hflag, base + (long long)F * sd, sd, cur);
         }
-        R prv[10];
+        R prv[NV];
 #pragma unroll
-        for (int m = 0; m < 10; m++) {
+        for (int m = 0; m < NV; m++) {
             R t = __shfl_up_sync(FULL, cur[m], LC);
             prv[m] = ly == 0 ? carry[m] : t;
             carry[m] = __shfl_sync(FULL, cur[m], (LY - 1) * LC + col);
@@ -179,8 +181,15 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep3(const __grid_constant_
         }
         if (valid && !defer) {
             R aj = (R)metric<UNI>(p, M_AJAC, base + (long long)F * sd);
-            if (DIR == 0) add_du<true>(du, N, ci, aj, h, ih, cur, prv, old);
-            else          add_du<false>(du, N, ci, aj, h, ih, cur, prv, old);
+            if constexpr (FAST) {
+                const R cf = up7_scale(aj, p.inv_h[DIR]);
+#pragma unroll
+                for (int m = 0; m < 5; m++)
+                    du[m * N + ci] = DIR == 0 ? cf * (cur[m] - prv[m]) : fma_r(cf, cur[m] - prv[m], old[m]);
+            } else {
+                if (DIR == 0) add_du<true>(du, N, ci, aj, h, ih, cur, prv, old);
+                else          add_du<false>(du, N, ci, aj, h, ih, cur, prv, old);
+            }
         }
         if (SYNC2) __syncwarp();
     }

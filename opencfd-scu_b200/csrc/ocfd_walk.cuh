@@ -195,6 +195,39 @@ __device__ __forceinline__ void face_up7(const R *ring, int col, int F, R (&out)
     }
 }
 
+// UP7 coefficients of the positive side, points F-3 .. F+4, times 420; the
+// negative side takes them mirrored (src/OCFD_Schemes.cu:865-907)
+template <typename R> __device__ __forceinline__ constexpr R up7_c(int k) {
+    return k == 0 ? (R)-3 : k == 1 ? (R)25 : k == 2 ? (R)-101 : k == 3 ? (R)319 : k == 4 ? (R)214
+         : k == 5 ? (R)-38 : k == 6 ? (R)4 : (R)0;
+}
+__device__ __forceinline__ double fma_r(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float fma_r(float a, float b, float c) { return fmaf(a, b, c); }
+
+// 420 times the sum of both signs' UP7 fluxes of face F+1/2.  A cell
+// between two UP7 faces needs no more than the difference of two such sums,
+// scaled once by -Ajac / (420 h): one product per field in place of twenty
+// quotients, and half the values to carry and to shuffle.  Point by point,
+// plus before minus, the order the marches add them in.
+template <int RING, int LC, typename R>
+__device__ __forceinline__ void face_up7_sum(const R *ring, int col, int F, R *out) {
+#pragma unroll
+    for (int m = 0; m < 5; m++) {
+        auto v = [&](int sv, int k) { return ring[(sv * RING + ((F - 3 + k) & (RING - 1))) * LC + col]; };
+        R s = up7_c<R>(0) * v(m, 0);
+#pragma unroll
+        for (int k = 1; k < 8; k++) {
+            if (k < 7) s = fma_r(up7_c<R>(k), v(m, k), s);
+            s = fma_r(up7_c<R>(7 - k), v(5 + m, k), s);
+        }
+        out[m] = s;
+    }
+}
+
+// -Ajac / (420 h)
+template <typename R>
+__device__ __forceinline__ R up7_scale(R aj, double inv_h) { return -aj * (R)(inv_h / 420.0); }
+
 
 // split of one point (primitives q5, LAP offset o) into ring slot P
 template <int DIR, int RING, int LC, bool UNI, bool EPS0, typename R>

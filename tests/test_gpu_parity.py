@@ -232,6 +232,10 @@ def _march_cases():
         ("rnd17x18x13_hybrid_char_curv_shock",
          cases.random_smooth_case(17, 18, 13, seed=65, scheme_invis="SCHEME_HYBRIDAUTO", charteric=1,
                                   shock=True, curvilinear=True)),
+        # one lane past a warp's columns; lines that split into segments with a short last one
+        ("rnd33x61x43_hybrid_char_curv",
+         cases.random_smooth_case(33, 61, 43, seed=12, scheme_invis="SCHEME_HYBRIDAUTO", charteric=1,
+                                  curvilinear=True)),
         ("rnd37x20x19_hybrid_char_shock",
          cases.random_smooth_case(37, 20, 19, seed=8, scheme_invis="SCHEME_HYBRIDAUTO", charteric=1, shock=True)),
     ]
@@ -241,9 +245,8 @@ def _march_cases():
 
 @pytest.mark.parametrize("name,case", _march_cases(), ids=[n for n, _ in _march_cases()])
 def test_march_matches_ring_walk(name, case, gpu_lib):
-    """The y and z UP7 walks run as per-lane marches over staged pencil tiles
-    (variant 8; variant 4 in the precision form) or through the shared-memory
-    ring (variant 7).  Same face and cell arithmetic and the same deferred
+    """The y and z UP7 walks run as per-lane marches (variants 4 and 8) or
+    through the shared-memory ring (variant 7).  Same face and cell arithmetic and the same deferred
     cells, so the same state to the last bit, in FP64 and in the precision
     form; and the FP64 state matches the in-loop dispatch (variant 5) to the
     walk-equivalence bound."""
