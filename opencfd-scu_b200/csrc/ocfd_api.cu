@@ -24,6 +24,7 @@ cudaError_t launch_q_criterion(const Params &p, double *q, cudaStream_t st);
 cudaError_t launch_time_average(const Params &p, double *mean5, int n, cudaStream_t st);
 bool march_supported(const Params &p, int dir);
 cudaError_t march_prepare();
+cudaError_t row_prepare();
 cudaError_t vdiv_prepare();
 cudaError_t launch_march_dir(const Params &p, int dir, cudaStream_t st);
 cudaError_t launch_ghost(const Params &p, double *const *fields, const int *dirmask, int nf, cudaStream_t st);
@@ -144,7 +145,6 @@ struct ocfd_b200_ctx {
     double walk4_threshold = 0.002;     // deferred cells per cell above which the inline walk is used
     // the UP7 walk of the y and z sweeps as per-lane marches (ocfd_march.cu);
     // 0: the shared-memory ring walk there too (sweep variant 7)
-    bool march_ok = false;      // the marches' shared-memory sizes are set
     bool vdiv_ok = true;        // the staged divergence kernel can be launched
     // running time averages of d, u, v, w, T (5 interior fields, allocated on
     // first use) and the number of samples in them
@@ -377,8 +377,11 @@ extern "C" int ocfd_b200_create(const ocfd_b200_config *cfg, ocfd_b200_ctx **out
     }
     // the staged divergence kernel is used only when its shared-memory size is set
     if (ocfd::vdiv_prepare() != cudaSuccess) { cudaGetLastError(); p.vis_impl = 1; ctx->vdiv_ok = false; }
-    ctx->march_ok = ocfd::march_prepare() == cudaSuccess;
-    cudaGetLastError();
+    if ((e = ocfd::march_prepare()) != cudaSuccess || (e = ocfd::row_prepare()) != cudaSuccess) {
+        cuda_fail(nullptr, e, "sweep kernels");
+        free_all(ctx); delete ctx;
+        return OCFD_ERR_CUDA;
+    }
 
     if ((e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreate(&ctx->ev[0])) != cudaSuccess || (e = cudaEventCreate(&ctx->ev[1])) != cudaSuccess ||
@@ -636,7 +639,7 @@ static int sweeps_auto(ocfd_b200_ctx *ctx) {
         if (w[d]) {
             CK(ocfd::launch_sweep4_dir(p, d, ctx->stream), "inviscid sweeps");
             ctx->launches += 1;
-        } else if (d > 0 && ctx->march && ctx->march_ok && ocfd::march_supported(p, d)) {
+        } else if (d > 0 && ctx->march && ocfd::march_supported(p, d)) {
             CK(ocfd::launch_march_dir(p, d, ctx->stream), "inviscid sweeps");
             ctx->launches += 2;
         } else {

@@ -16,6 +16,7 @@
 namespace ocfd {
 
 cudaError_t launch_sweep4_fix(const Params &p, int dir, cudaStream_t st);
+cudaError_t launch_row(const Params &p, cudaStream_t st);
 
 namespace {
 
@@ -355,6 +356,8 @@ __global__ void __launch_bounds__(32 * FIXW) k_sweep3_fix(const __grid_constant_
 
 template <int DIR, bool UNI, bool EPS0, int MINB, bool FAST, typename R = double>
 cudaError_t launch_dir(const Params &p, cudaStream_t st) {
+    if constexpr (FAST && DIR == 0) return launch_row(p, st);      // ocfd_row.cu
+    else {
     constexpr int LC = Shape<DIR>::LC, LY = 32 / LC;
     const int n = DIR == 0 ? p.nx : (DIR == 1 ? p.ny : p.nz);
     const long long ngx = (p.nx + LC - 1) / LC;
@@ -379,6 +382,7 @@ cudaError_t launch_dir(const Params &p, cudaStream_t st) {
     // that strides over it (usually a few thousand cells, often none)
     k_sweep3_fix<DIR, UNI, EPS0><<<2 * 148, 32 * FIXW, 0, st>>>(p);
     return cudaGetLastError();
+    }
 }
 
 template <bool UNI, bool EPS0, int MINB, bool FAST>

@@ -270,6 +270,31 @@ def test_march_matches_ring_walk(name, case, gpu_lib):
             assert np.all(rel_l2(a.primitives(), c.primitives()) <= 1e-14), name
 
 
+@pytest.mark.parametrize("nx", [8, 31, 33, 64, 97, 132, 161])
+@pytest.mark.parametrize("curvilinear,closed", [(False, False), (True, True)])
+def test_row_walk_widths(nx, curvilinear, closed, gpu_lib):
+    """The x walk takes 8, 16 or 32 lanes a row by the row's width and
+    16-byte stores where it is a multiple of four: every choice, with ragged last
+    passes and rows left over, against the in-loop dispatch (the same bound
+    as the other walks)."""
+    case = cases.random_smooth_case(nx, 11, 9, seed=nx, scheme_invis="SCHEME_HYBRIDAUTO", charteric=1,
+                                    shock=nx == 97, curvilinear=curvilinear,
+                                    iperiodic=(0, 1, 1) if closed else (1, 1, 1),
+                                    dif_bound=(1, 1, 0, 0, 0, 0) if closed else (0,) * 6)
+    a = lib.Solver(case.cfg, case.prims, case.metrics)
+    a.set_walk_threshold(3.0)
+    b = lib.Solver(case.cfg, case.prims, case.metrics)
+    b.set_sweep_impl(5)
+    f = lib.Solver(case.cfg, case.prims, case.metrics)
+    f.set_walk_threshold(3.0)
+    f.set_precision(1)
+    for s in (a, b, f):
+        s.step(2)
+    assert a.sweep_walks() == 0
+    assert np.all(rel_l2(a.primitives(), b.primitives()) <= 1e-14)
+    assert np.all(rel_l2(f.conserved(), b.conserved()) <= 2e-5)        # the precision form's bound
+
+
 def _viscous_cases():
     """Viscous-kernel cases: CD6 and CD8, uniform and curvilinear metrics,
     closed faces, a width that is not a multiple of the 32-cell tile, the
