@@ -38,7 +38,8 @@ cudaError_t launch_rk(const Params &p, int krk, cudaStream_t st);
 cudaError_t launch_rk_only(const Params &p, int krk, cudaStream_t st);
 cudaError_t launch_c2p(const Params &p, cudaStream_t st);
 cudaError_t launch_bc_faces(const Params &p, cudaStream_t st);
-cudaError_t launch_p2c(const Params &p, double *out, cudaStream_t st);
+cudaError_t launch_load_state(const Params &p, const double *src, bool wrap, bool f32, cudaStream_t st);
+cudaError_t launch_store_state(const Params &p, double *out, bool from_f, cudaStream_t st);
 cudaError_t launch_scatter(const Params &p, const double *src, double *dst_lap, cudaStream_t st);
 cudaError_t launch_gather(const Params &p, const double *src_lap, double *dst, cudaStream_t st);
 cudaError_t launch_fill(double *f, long long n, double v, cudaStream_t st);
@@ -1208,32 +1209,36 @@ extern "C" int ocfd_b200_set_mesh_device(ocfd_b200_ctx *ctx, const double *xyz3_
     return set_mesh_impl(ctx, xyz3_dev, cudaMemcpyDeviceToDevice);
 }
 
-static int upload_prims(ocfd_b200_ctx *ctx, const double *src, cudaMemcpyKind kind) {
-    const Params &p = ctx->p;
-    size_t inB = sizeof(double) * (size_t)p.N;
-    CK(cudaMemcpyAsync(ctx->stage_buf, src, 5 * inB, kind, ctx->stream), "primitive copy");
-    for (int m = 0; m < 5; m++) {
-        CK(ocfd::launch_scatter(p, ctx->stage_buf + (size_t)m * p.N, p.prim[m], ctx->stream), "scatter");
-        ctx->launches += 1;
-    }
-    return OCFD_OK;
+// The caller's device array can be read in place: aligned memory of this
+// GPU outside the context's own conserved fields (which the load overwrites).
+// Anything else goes through the staging copy.
+static bool reads_in_place(const ocfd_b200_ctx *ctx, const double *src) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, src) != cudaSuccess) { cudaGetLastError(); return false; }
+    if (a.type != cudaMemoryTypeDevice || a.device != ctx->device || (reinterpret_cast<uintptr_t>(src) & 7)) return false;
+    const double *c = ctx->cons_buf, *q = ctx->prim_buf;
+    const size_t N = (size_t)ctx->p.N, lapN = (size_t)ctx->p.lapN;
+    return (src + 5 * N <= c || src >= c + 15 * N) && (src + 5 * N <= q || src >= q + 5 * lapN);
 }
 
 static int set_prims_impl(ocfd_b200_ctx *ctx, const double *src, cudaMemcpyKind kind, int istep, double tt) {
     if (!ctx || !src) return OCFD_ERR_ARG;
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     const Params &p = ctx->p;
-    // init(): ghosts of d,u,v,w,T zero (src/OCFD_init.cu:37-41), f/fn/du zero
-    CK(cudaMemsetAsync(ctx->prim_buf, 0, 5 * sizeof(double) * (size_t)p.lapN, ctx->stream), "memset");
-    CK(cudaMemsetAsync(ctx->cons_buf, 0, 15 * sizeof(double) * (size_t)p.N, ctx->stream), "memset");
-    int rc = upload_prims(ctx, src, kind);
-    if (rc) return rc;
-    CK(ocfd::launch_p2c(p, p.f, ctx->stream), "pri_to_cons");
-    ctx->launches += 1;
+    const size_t inB = sizeof(double) * (size_t)p.N;
+    if (kind == cudaMemcpyHostToDevice || !reads_in_place(ctx, src)) {
+        CK(cudaMemcpyAsync(ctx->stage_buf, src, 5 * inB, kind, ctx->stream), "primitive copy");
+        src = ctx->stage_buf;
+    }
+    // init(): ghosts of d,u,v,w,T zero (src/OCFD_init.cu:37-41), f from them, fn/du zero.
     // NS_solver_real pre-loop: exchange, OCFD_bc (the boundary family's
     // values, then the faces of f re-projected: without a family no change),
-    // get_Amu (formed on the fly)
-    rc = ghost_prims64(ctx);
+    // get_Amu (formed on the fly).  On one GPU the load fills the periodic
+    // ghosts itself; the boundary family's values come before the FP32 ones.
+    const bool f32 = p.mixed && !p.ibc && !ctx->slab;
+    CK(ocfd::launch_load_state(p, src, !ctx->slab, f32, ctx->stream), "state load");
+    ctx->launches += 1;
+    int rc = ctx->slab ? ghost_prims64(ctx) : OCFD_OK;
     if (rc) return rc;
     ctx->tt = tt;
     if (p.ibc) {
@@ -1241,7 +1246,7 @@ static int set_prims_impl(ocfd_b200_ctx *ctx, const double *src, cudaMemcpyKind 
         CK(ocfd::launch_bc_faces(p, ctx->stream), "face re-projection");
         ctx->launches += 1;
     }
-    if (p.mixed) {
+    if (p.mixed && !f32) {
         CK(ocfd::launch_prims_to_fp32(p, ctx->stream), "FP32 primitives");
         ctx->launches += 1;
     }
@@ -1645,14 +1650,20 @@ extern "C" int ocfd_b200_bc(ocfd_b200_ctx *ctx) {
 // read-back
 // ---------------------------------------------------------------------------
 
+// the dense primitives into device memory (in the precision form the
+// interior alone is brought up to date: its ghosts wait for a reader)
+static int store_prims(ocfd_b200_ctx *ctx, double *out) {
+    const bool from_f = ctx->prims64_stale && !ctx->prims64_interior_ok;
+    CK(ocfd::launch_store_state(ctx->p, out, from_f, ctx->stream), "state store");
+    ctx->launches += 1;
+    if (from_f) ctx->prims64_interior_ok = true;
+    return OCFD_OK;
+}
+
 extern "C" int ocfd_b200_get_primitives_device(ocfd_b200_ctx *ctx, double *out) {
     if (!ctx || !out) return OCFD_ERR_ARG;
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
-    if (int rc = refresh_prims64(ctx)) return rc;
-    for (int m = 0; m < 5; m++) {
-        CK(ocfd::launch_gather(ctx->p, ctx->p.prim[m], out + (size_t)m * ctx->p.N, ctx->stream), "gather");
-        ctx->launches += 1;
-    }
+    if (int rc = store_prims(ctx, out)) return rc;
     CK(cudaStreamSynchronize(ctx->stream), "get_primitives");
     return OCFD_OK;
 }
@@ -1660,11 +1671,7 @@ extern "C" int ocfd_b200_get_primitives_device(ocfd_b200_ctx *ctx, double *out) 
 extern "C" int ocfd_b200_get_primitives(ocfd_b200_ctx *ctx, double *out) {
     if (!ctx || !out) return OCFD_ERR_ARG;
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
-    if (int rc = refresh_prims64(ctx)) return rc;
-    for (int m = 0; m < 5; m++) {
-        CK(ocfd::launch_gather(ctx->p, ctx->p.prim[m], ctx->stage_buf + (size_t)m * ctx->p.N, ctx->stream), "gather");
-        ctx->launches += 1;
-    }
+    if (int rc = store_prims(ctx, ctx->stage_buf)) return rc;
     CK(cudaMemcpyAsync(out, ctx->stage_buf, 5 * sizeof(double) * (size_t)ctx->p.N, cudaMemcpyDeviceToHost,
                        ctx->stream), "primitive copy");
     CK(cudaStreamSynchronize(ctx->stream), "get_primitives");

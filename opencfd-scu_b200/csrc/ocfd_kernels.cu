@@ -919,22 +919,6 @@ __global__ void k_bc_faces(Params p) {
     p.f[4 * N + tid] = d * ((u * u + v * v + w * w) * 0.5 + p.Cv * T);
 }
 
-// pri_to_cons over the interior (init, src/OCFD_init.cu:108-115)
-__global__ void k_p2c(Params p, double *out) {
-    long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid >= p.N) return;
-    int i = (int)(tid % p.nx); long long r = tid / p.nx;
-    int j = (int)(r % p.ny); int k = (int)(r / p.ny);
-    long long o = lap_index(p, i + OCFD_LAP, j + OCFD_LAP, k + OCFD_LAP);
-    double d = p.prim[0][o], u = p.prim[1][o], v = p.prim[2][o], w = p.prim[3][o], T = p.prim[4][o];
-    const long long N = p.N;
-    out[tid] = d;
-    out[N + tid] = u * d;
-    out[2 * N + tid] = v * d;
-    out[3 * N + tid] = w * d;
-    out[4 * N + tid] = d * ((u * u + v * v + w * w) * 0.5 + p.Cv * T);
-}
-
 // interior <-> LAP-box copy of one field (dense [nz][ny][nx] <-> LAP box)
 __global__ void k_scatter_interior(Params p, const double *src, double *dst_lap) {
     long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -950,6 +934,80 @@ __global__ void k_gather_interior(Params p, const double *src_lap, double *dst) 
     int j = (int)(r % p.ny); int k = (int)(r / p.ny);
     dst[tid] = src_lap[lap_index(p, i + OCFD_LAP, j + OCFD_LAP, k + OCFD_LAP)];
 }
+// A whole state from the caller's dense primitives (init,
+// src/OCFD_init.cu:37-41,108-115, and the exchange before the loop,
+// src/OCFD_mpi_dev.cu:186-310), one thread per element of the LAP box:
+// the interior's primitives and f, fn and du zero; with wrap the periodic
+// ghosts from the cells they repeat (else zero, as every other ghost and the
+// row padding); with f32 the precision form's primitives too.  Bound by
+// DRAM: every value is read once and written once where a copy, two fills,
+// five copies into the LAP box, a conversion to f, the ghost fill and the
+// FP32 conversion each made a pass of their own.  With the one-pass read-back
+// below, a 256^3 run of two steps in the precision form takes 12.44 ms where
+// it took 13.61, a 16^3 step 214 us where it took 260.
+__global__ void __launch_bounds__(256) k_load_state(Params p, const double *__restrict__ src, int wrap, int f32) {
+    const int ntx = (int)((p.ys + 31) / 32), nyl = p.ny + 2 * OCFD_LAP;
+    const int il = (int)(blockIdx.x % ntx) * 32 + (int)(threadIdx.x % 32);
+    const int jl = (int)(blockIdx.x / ntx) * 8 + (int)(threadIdx.x / 32);
+    const int kl = (int)blockIdx.y;
+    if (il >= p.ys || jl >= nyl) return;
+    const long long o = OCFD_IDX(p, (long long)il + p.ys * jl + p.zs * kl, p.lapN), N = p.N;
+    int i = il - OCFD_LAP, j = jl - OCFD_LAP, k = kl - OCFD_LAP;
+    const bool gx = i < 0 || i >= p.nx, gy = j < 0 || j >= p.ny, gz = k < 0 || k >= p.nz;
+    double q[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    const bool ghost = wrap && i < p.nx + OCFD_LAP && (int)gx + (int)gy + (int)gz == 1 &&
+                       ((gx && p.periodic[0]) || (gy && p.periodic[1]) || (gz && p.periodic[2]));
+    const bool inner = !gx && !gy && !gz;
+    if (inner || ghost) {
+        i += i < 0 ? p.nx : i >= p.nx ? -p.nx : 0;
+        j += j < 0 ? p.ny : j >= p.ny ? -p.ny : 0;
+        k += k < 0 ? p.nz : k >= p.nz ? -p.nz : 0;
+        const long long c = in_index(p, i, j, k);
+#pragma unroll
+        for (int m = 0; m < 5; m++) q[m] = src[m * N + c];
+        if (inner) {
+            const double d = q[0], u = q[1], v = q[2], w = q[3], T = q[4];
+            p.f[c] = d;
+            p.f[N + c] = u * d;
+            p.f[2 * N + c] = v * d;
+            p.f[3 * N + c] = w * d;
+            p.f[4 * N + c] = d * ((u * u + v * v + w * w) * 0.5 + p.Cv * T);
+#pragma unroll
+            for (int m = 0; m < 5; m++) { p.fn[m * N + c] = 0.0; p.du[m * N + c] = 0.0; }
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < 5; m++) {
+        p.prim[m][o] = q[m];
+        if (f32) p.prim32[m][o] = (float)q[m];
+    }
+}
+
+// The dense primitives of the state; with from_f (precision form, interior
+// not formed since the last step) they are formed from f first, as k_c2p
+// forms them.
+__global__ void __launch_bounds__(256) k_store_state(Params p, double *__restrict__ out, int from_f) {
+    const int ntx = (p.nx + 31) / 32;
+    const int i = (int)(blockIdx.x % ntx) * 32 + (int)(threadIdx.x % 32);
+    const int j = (int)(blockIdx.x / ntx) * 8 + (int)(threadIdx.x / 32);
+    const int k = (int)blockIdx.y;
+    if (i >= p.nx || j >= p.ny) return;
+    const long long o = lap_index(p, i + OCFD_LAP, j + OCFD_LAP, k + OCFD_LAP), c = in_index(p, i, j, k), N = p.N;
+    double q[5];
+    if (from_f) {
+        const double f[5] = {p.f[c], p.f[N + c], p.f[2 * N + c], p.f[3 * N + c], p.f[4 * N + c]};
+        cons_to_prim(p, f, q[0], q[1], q[2], q[3], q[4]);
+#pragma unroll
+        for (int m = 0; m < 5; m++) p.prim[m][o] = q[m];
+        if (p.pfil) p.pfil[o] = q[4] * q[0] / (p.Gamma * p.Ama * p.Ama);
+    } else {
+#pragma unroll
+        for (int m = 0; m < 5; m++) q[m] = p.prim[m][o];
+    }
+#pragma unroll
+    for (int m = 0; m < 5; m++) out[m * N + c] = q[m];
+}
+
 // the FP32 primitives of the precision form from the FP64 ones (whole LAP box)
 __global__ void k_prims_to_fp32(Params p) {
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1223,8 +1281,15 @@ cudaError_t launch_rk(const Params &p, int krk, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_p2c(const Params &p, double *out, cudaStream_t st) {
-    k_p2c<<<blocks_for(p.N, 256), 256, 0, st>>>(p, out);
+cudaError_t launch_load_state(const Params &p, const double *src, bool wrap, bool f32, cudaStream_t st) {
+    const dim3 grid((unsigned)((p.ys + 31) / 32 * ((p.ny + 2 * OCFD_LAP + 7) / 8)), (unsigned)(p.nz + 2 * OCFD_LAP));
+    k_load_state<<<grid, 256, 0, st>>>(p, src, wrap ? 1 : 0, f32 ? 1 : 0);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_store_state(const Params &p, double *out, bool from_f, cudaStream_t st) {
+    const dim3 grid((unsigned)((p.nx + 31) / 32 * ((p.ny + 7) / 8)), (unsigned)p.nz);
+    k_store_state<<<grid, 256, 0, st>>>(p, out, from_f ? 1 : 0);
     return cudaGetLastError();
 }
 

@@ -419,3 +419,41 @@ def test_per_stage_api_equals_step_with_bc_and_filter(gpu_lib):
         assert b.L.ocfd_b200_filtering(b.h) == 0
     assert np.array_equal(a.primitives(), b.primitives())
     assert np.array_equal(a.conserved(), b.conserved())
+
+
+@pytest.mark.parametrize("dims", [(8, 9, 33), (41, 8, 10), (33, 17, 8)])
+@pytest.mark.parametrize("form", [0, 1])
+def test_state_load_and_store(gpu_lib, dims, form):
+    """Whole states from host memory, and from device memory in place (also
+    one element off the allocation's alignment): the same primitives back,
+    the same conserved state, the same step.  In the precision form a
+    read-back (which forms the interior alone) before another reader leaves
+    that reader's result as it is without it."""
+    import torch
+
+    case = cases.random_smooth_case(*dims, seed=11, scheme_invis="WENO7", curvilinear=True)
+    q = np.stack(case.prims)
+    runs = []
+    for src in ("host", "device", "offset"):
+        s = lib.Solver(case.cfg, case.prims, case.metrics)
+        if form:
+            s.set_precision(1)
+        s.step(1)                               # leaves fn, du and the ghosts in use
+        if src in ("device", "offset"):
+            buf = torch.zeros(q.size + 1, dtype=torch.float64, device="cuda")
+            t = buf[int(src == "offset"):][:q.size]
+            t.copy_(torch.from_numpy(q).flatten())
+            torch.cuda.synchronize()
+            s.set_primitives_device(t.data_ptr())
+        else:
+            s.set_primitives(case.prims)
+        assert np.array_equal(s.primitives(), q)
+        u = s.conserved()
+        assert np.array_equal(u[0], q[0]) and np.array_equal(u[2], q[2] * q[0])
+        s.step(1)
+        if src == "device":
+            s.primitives()                      # the interior first, the ghosts with the next reader
+        runs.append((u, s.q_criterion(), s.conserved(), s.primitives()))
+        s.close()
+    for r in runs[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(r, runs[0]))
