@@ -258,6 +258,15 @@ static void free_all(ocfd_b200_ctx *c) {
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
 }
 
+// divisors of the viscous scheme's differences (CD6: 60 h, CD8: 840 h)
+static void set_d0(Params &p) {
+    const double h[3] = { p.hx, p.hy, p.hz }, c = p.scheme_vis == 204 ? 840.0 : 60.0;
+    for (int d = 0; d < 3; d++) {
+        p.d0_h[d] = c * h[d];
+        p.d0_ih[d] = 1.0 / p.d0_h[d];
+    }
+}
+
 extern "C" int ocfd_b200_create(const ocfd_b200_config *cfg, ocfd_b200_ctx **out) {
     ocfd_b200_ctx *ctx = nullptr;
     if (!cfg || !out) return fail(nullptr, OCFD_ERR_ARG, "null argument");
@@ -318,6 +327,7 @@ extern "C" int ocfd_b200_create(const ocfd_b200_config *cfg, ocfd_b200_ctx **out
     p.nochar_comp_flag = cfg->hybrid_nochar_same_flag ? 0 : 3;
     p.sweep_impl = 4;
     p.inv_h[0] = 1.0 / p.hx; p.inv_h[1] = 1.0 / p.hy; p.inv_h[2] = 1.0 / p.hz;
+    set_d0(p);
     p.inv_Ama = 1.0 / Ma;
     for (int d = 0; d < 3; d++) p.periodic[d] = cfg->iperiodic[d];
     p.zface_lo = p.zface_hi = 1;
@@ -872,6 +882,7 @@ static int set_slab_impl(ocfd_b200_ctx *ctx, int nranks, int rank, int rank_lo, 
     // only the faces of the whole grid (src/OCFD_boundary.cu:78-95)
     p.hz = 1.0 / (nz_global - 1.0);
     p.inv_h[2] = 1.0 / p.hz;
+    set_d0(p);
     p.zface_lo = z_offset == 0;
     p.zface_hi = z_offset + p.nz == nz_global;
     // z closures (DIF_BOUND, NON_REFLETION) act at the faces of the whole

@@ -62,6 +62,7 @@ struct Params {
     double mc[13];
     DirConst dc[3];
     double inv_h[3], inv_Ama;   // reciprocals for div_const
+    double d0_h[3], d0_ih[3];   // divisor of the viscous scheme's difference (60 h or 840 h) and its reciprocal
     int sweep_impl;         // 4: the walks chosen per direction (default); 5: every face through the in-loop dispatch; 6: the in-line walk
     // viscous divergence + RK of whole steps: 0 Ev tiles staged in shared
     // memory in the precision form, read through L1/L2 in FP64 (each the
@@ -523,13 +524,13 @@ __device__ __forceinline__ double symbo_m(int lmt, double tv_lim, double tv_max,
     return symbo_core(TVmax < tv_lim*TVmin && TVmax < tv_max, v);
 }
 
-// CD6 / CD8 first derivative, src/OCFD_Schemes.cu:96-126
+// CD6 / CD8 first difference, 60 h or 840 h times the derivative, src/OCFD_Schemes.cu:96-126
 __device__ __forceinline__ double cd6(double sm3, double sm2, double sm1, double sp1, double sp2, double sp3) {
-    return (45.0*(sp1 - sm1) - 9.0*(sp2 - sm2) + (sp3 - sm3))/60.0;
+    return 45.0*(sp1 - sm1) - 9.0*(sp2 - sm2) + (sp3 - sm3);
 }
 __device__ __forceinline__ double cd8(double sm4, double sm3, double sm2, double sm1,
                                       double sp1, double sp2, double sp3, double sp4) {
-    return (672.0*(sp1 - sm1) - 168.0*(sp2 - sm2) + 32.0*(sp3 - sm3) - 3.0*(sp4 - sm4))/840.0;
+    return 672.0*(sp1 - sm1) - 168.0*(sp2 - sm2) + 32.0*(sp3 - sm3) - 3.0*(sp4 - sm4);
 }
 
 // ---------------------------------------------------------------------------

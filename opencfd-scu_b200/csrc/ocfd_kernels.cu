@@ -166,24 +166,34 @@ cudaError_t compute_dirconst(Params &p, DirConst *dev_scratch, cudaStream_t st) 
 // viscous terms, src/OCFD_NS_Jacobian3d.cu:58-440
 // ---------------------------------------------------------------------------
 
+// divisors of a direction's derivative: h (closures) and the scheme's 60 h or 840 h
+template <typename R> struct D0 {
+    R h, ih, hq, ihq;
+    __device__ __forceinline__ D0(const Params &p, int d)
+        : h((R)(d == 0 ? p.hx : d == 1 ? p.hy : p.hz)), ih((R)p.inv_h[d]), hq((R)p.d0_h[d]), ihq((R)p.d0_ih[d]) {}
+};
+
 // first derivative of a LAP field along stride s at o (OCFD_d?0 with CD6 or
-// CD8, src/OCFD_Schemes.cu:96-156; put_d0_kernel divides by h)
-// (the division by h is the corrected product with RN(1/h), div_const)
-template <typename R>
-__device__ __forceinline__ R d0(const R *f, long long o, long long s, R h, R ih, bool c8) {
+// CD8, src/OCFD_Schemes.cu:96-156; put_d0_kernel divides by h).  The two
+// quotients are one, by 60 h or 840 h, formed as the corrected product with
+// its reciprocal (div_const): the division by 60 was the larger part of a
+// derivative's instructions.
+template <bool C8, typename R>
+__device__ __forceinline__ R d0(const R *f, long long o, long long s, const D0<R> &c) {
     R t;
-    if (c8) t = cd8(f[o - 4 * s], f[o - 3 * s], f[o - 2 * s], f[o - s], f[o + s], f[o + 2 * s], f[o + 3 * s], f[o + 4 * s]);
+    if (C8) t = cd8(f[o - 4 * s], f[o - 3 * s], f[o - 2 * s], f[o - s], f[o + s], f[o + 2 * s], f[o + 3 * s], f[o + 4 * s]);
     else    t = cd6(f[o - 3 * s], f[o - 2 * s], f[o - s], f[o + s], f[o + 2 * s], f[o + 3 * s]);
-    return div_const(t, h, ih);
+    return div_const(t, c.hq, c.ihq);
 }
 
 // The same derivative at point X of a line of n cells whose faces may be
 // closed (DIF_BOUND = 1): the one-sided and lower-order formulas of
 // OCFD_D0bound_scheme_kernel (src/OCFD_bound_Scheme.cu:79-186) on the four
 // points next to a closed face, the lower face first as in its case 7/8/9.
-template <typename R>
-__device__ __forceinline__ R d0b(const R *f, long long o, long long s, R h, R ih, bool c8,
+template <bool C8, typename R>
+__device__ __forceinline__ R d0b(const R *f, long long o, long long s, const D0<R> &c,
                                  int X, int n, bool lo, bool hi) {
+    const R h = c.h, ih = c.ih;
     if (lo && X <= 3) {
         R t;
         if (X == 0)      t = (f[o + s] - f[o]);
@@ -203,7 +213,7 @@ __device__ __forceinline__ R d0b(const R *f, long long o, long long s, R h, R ih
                               + (R)45.0 * (f[o + s] - f[o - s])) / (R)60.0;
         return div_const(t, h, ih);
     }
-    return d0(f, o, s, h, ih, c8);
+    return d0<C8>(f, o, s, c);
 }
 
 // cons_to_pri of one cell (src/commen_kernel.cu:77-109): one reciprocal of
@@ -237,39 +247,28 @@ __device__ __forceinline__ bool tile_cell(const Params &p, int &i, int &j, int &
 // and temperature derivatives (du_viscous_Jacobian3d_init :58-77) are formed
 // here from the LAP-box primitives instead of being stored; the stress and
 // heat flux do not depend on the direction, so they are formed once per cell.
-template <bool UNI, typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 8 ? 5 : 6) k_vis_ev(Params p) {
+// Bound by the latency of its 72 stencil loads: without a branch on the scheme
+// or the closures between them a cell's loads go out together, and 64
+// registers (4 blocks an SM) hold them.  256^3: 770 -> 592 us (5 blocks 642, 3
+// 624); ramp 512x128x64 367 -> 268 us (5 and 3 blocks 322).
+template <bool UNI, bool BND, bool C8, typename R>
+__global__ void __launch_bounds__(256, sizeof(R) == 8 ? 4 : 6) k_vis_ev(const __grid_constant__ Params p) {
     int i, j, k;
     long long tid;
     if (!tile_cell(p, i, j, k, tid)) return;
     long long o = lap_index(p, i + OCFD_LAP, j + OCFD_LAP, k + OCFD_LAP);
-    const bool c8 = p.scheme_vis == 204;
     R Akx = (R)metric<UNI>(p, M_AKX, o), Aix = (R)metric<UNI>(p, M_AIX, o), Asx = (R)metric<UNI>(p, M_ASX, o);
     R Aky = (R)metric<UNI>(p, M_AKY, o), Aiy = (R)metric<UNI>(p, M_AIY, o), Asy = (R)metric<UNI>(p, M_ASY, o);
     R Akz = (R)metric<UNI>(p, M_AKZ, o), Aiz = (R)metric<UNI>(p, M_AIZ, o), Asz = (R)metric<UNI>(p, M_ASZ, o);
     const R *U = prim_r<R>(p, 1), *V = prim_r<R>(p, 2), *W = prim_r<R>(p, 3), *TT = prim_r<R>(p, 4);
     R Tc = TT[o];
     R Amu = (R)p.amu_C0 * sqrt_r(Tc * Tc * Tc) / ((R)p.Tsb + Tc);      // get_Amu_kernal
-    const R ihx = (R)p.inv_h[0], ihy = (R)p.inv_h[1], ihz = (R)p.inv_h[2];
-    const R hx = (R)p.hx, hy = (R)p.hy, hz = (R)p.hz;
-    R uk, ui, us, vk, vi, vs, wk, wi, ws, Tk, Ti, Ts;
-    if (!p.has_bnd) {
-        uk = d0(U, o, 1, hx, ihx, c8); ui = d0(U, o, p.ys, hy, ihy, c8); us = d0(U, o, p.zs, hz, ihz, c8);
-        vk = d0(V, o, 1, hx, ihx, c8); vi = d0(V, o, p.ys, hy, ihy, c8); vs = d0(V, o, p.zs, hz, ihz, c8);
-        wk = d0(W, o, 1, hx, ihx, c8); wi = d0(W, o, p.ys, hy, ihy, c8); ws = d0(W, o, p.zs, hz, ihz, c8);
-        Tk = d0(TT, o, 1, hx, ihx, c8); Ti = d0(TT, o, p.ys, hy, ihy, c8); Ts = d0(TT, o, p.zs, hz, ihz, c8);
-    } else {
-        const bool bxl = p.bnd_lo[0], bxh = p.bnd_hi[0], byl = p.bnd_lo[1], byh = p.bnd_hi[1];
-        const bool bzl = p.bnd_lo[2], bzh = p.bnd_hi[2];
-        uk = d0b(U, o, 1, hx, ihx, c8, i, p.nx, bxl, bxh); ui = d0b(U, o, p.ys, hy, ihy, c8, j, p.ny, byl, byh);
-        us = d0b(U, o, p.zs, hz, ihz, c8, k, p.nz, bzl, bzh);
-        vk = d0b(V, o, 1, hx, ihx, c8, i, p.nx, bxl, bxh); vi = d0b(V, o, p.ys, hy, ihy, c8, j, p.ny, byl, byh);
-        vs = d0b(V, o, p.zs, hz, ihz, c8, k, p.nz, bzl, bzh);
-        wk = d0b(W, o, 1, hx, ihx, c8, i, p.nx, bxl, bxh); wi = d0b(W, o, p.ys, hy, ihy, c8, j, p.ny, byl, byh);
-        ws = d0b(W, o, p.zs, hz, ihz, c8, k, p.nz, bzl, bzh);
-        Tk = d0b(TT, o, 1, hx, ihx, c8, i, p.nx, bxl, bxh); Ti = d0b(TT, o, p.ys, hy, ihy, c8, j, p.ny, byl, byh);
-        Ts = d0b(TT, o, p.zs, hz, ihz, c8, k, p.nz, bzl, bzh);
-    }
+    const D0<R> cx(p, 0), cy(p, 1), cz(p, 2);
+    auto dx = [&](const R *f) { return BND ? d0b<C8>(f, o, 1, cx, i, p.nx, p.bnd_lo[0], p.bnd_hi[0]) : d0<C8>(f, o, 1, cx); };
+    auto dy = [&](const R *f) { return BND ? d0b<C8>(f, o, p.ys, cy, j, p.ny, p.bnd_lo[1], p.bnd_hi[1]) : d0<C8>(f, o, p.ys, cy); };
+    auto dz = [&](const R *f) { return BND ? d0b<C8>(f, o, p.zs, cz, k, p.nz, p.bnd_lo[2], p.bnd_hi[2]) : d0<C8>(f, o, p.zs, cz); };
+    const R uk = dx(U), ui = dy(U), us = dz(U), vk = dx(V), vi = dy(V), vs = dz(V);
+    const R wk = dx(W), wi = dy(W), ws = dz(W), Tk = dx(TT), Ti = dy(TT), Ts = dz(TT);
     R ux = uk*Akx + ui*Aix + us*Asx;
     R vx = vk*Akx + vi*Aix + vs*Asx;
     R wx = wk*Akx + wi*Aix + ws*Asx;
@@ -387,16 +386,17 @@ __device__ __forceinline__ void rk_cell(const Params &p, int krk, long long tid,
 // (du_viscous_Jacobian3d_{x,y,z}_final + YF_Pe_XF, src/commen_kernel.cu:158-169).
 // RK = true: the stage's du is complete here, so the RK update, cons->prim
 // and the face re-projection follow in the same thread and du is not stored.
-template <bool UNI, bool RK, typename R>
-__global__ void __launch_bounds__(256, 6) k_vis_div(Params p, int krk, int k0) {
+// Bound by DRAM and the latency of its 82 loads, which 80 registers (3 blocks
+// an SM) keep in flight together where no closure branches part them.  256^3:
+// 1077 -> 932 us (6 blocks 994, 4 955); with closures 6 blocks (ramp
+// 512x128x64 276 us; 4 324, 3 321).
+template <bool UNI, bool BND, bool C8, bool RK, typename R>
+__global__ void __launch_bounds__(256, BND || sizeof(R) == 4 ? 6 : 3) k_vis_div(const __grid_constant__ Params p, int krk, int k0) {
     int i, j, k;
     long long tid;
     if (!tile_cell(p, i, j, k, tid, k0)) return;
     long long o = lap_index(p, i + OCFD_LAP, j + OCFD_LAP, k + OCFD_LAP);
     const long long st[3] = { 1LL, p.ys, p.zs };
-    const R hh[3] = { (R)p.hx, (R)p.hy, (R)p.hz };
-    const R ihh[3] = { (R)p.inv_h[0], (R)p.inv_h[1], (R)p.inv_h[2] };
-    const bool c8 = p.scheme_vis == 204;
     const R ajac = (R)metric<UNI>(p, M_AJAC, o);
     R *const du = du_r<R>(p);
     const R *const evb = ev_r<R>(p);
@@ -408,11 +408,11 @@ __global__ void __launch_bounds__(256, 6) k_vis_div(Params p, int krk, int k0) {
 #pragma unroll
         for (int m = 0; m < 4; m++) {
             const R *f = evb + (long long)(4 * dd + m) * p.lapN;
-            if (!p.has_bnd) {
-                acc[m + 1] += ajac * d0(f, o, st[dd], hh[dd], ihh[dd], c8);
+            if (!BND) {
+                acc[m + 1] += ajac * d0<C8>(f, o, st[dd], D0<R>(p, dd));
             } else {
                 const int X = dd == 0 ? i : (dd == 1 ? j : k), n = dd == 0 ? p.nx : (dd == 1 ? p.ny : p.nz);
-                acc[m + 1] += ajac * d0b(f, o, st[dd], hh[dd], ihh[dd], c8, X, n, p.bnd_lo[dd], p.bnd_hi[dd]);
+                acc[m + 1] += ajac * d0b<C8>(f, o, st[dd], D0<R>(p, dd), X, n, p.bnd_lo[dd], p.bnd_hi[dd]);
             }
         }
     }
@@ -452,14 +452,15 @@ struct VdivTiles {
 
 // d0 / d0b of k_vis_div from a window v[0..2H] (v[H] the cell), same expressions
 template <typename R, int H>
-__device__ __forceinline__ R d0w(const R *v, R h, R ih, bool c8) {
+__device__ __forceinline__ R d0w(const R *v, const D0<R> &c) {
     R t;
-    if (c8) t = cd8(v[H - 4], v[H - 3], v[H - 2], v[H - 1], v[H + 1], v[H + 2], v[H + 3], v[H + 4]);
-    else    t = cd6(v[H - 3], v[H - 2], v[H - 1], v[H + 1], v[H + 2], v[H + 3]);
-    return div_const(t, h, ih);
+    if constexpr (H == 4) t = cd8(v[H - 4], v[H - 3], v[H - 2], v[H - 1], v[H + 1], v[H + 2], v[H + 3], v[H + 4]);
+    else t = cd6(v[H - 3], v[H - 2], v[H - 1], v[H + 1], v[H + 2], v[H + 3]);
+    return div_const(t, c.hq, c.ihq);
 }
 template <typename R, int H>
-__device__ __forceinline__ R d0bw(const R *v, R h, R ih, bool c8, int X, int n, bool lo, bool hi) {
+__device__ __forceinline__ R d0bw(const R *v, const D0<R> &c, int X, int n, bool lo, bool hi) {
+    const R h = c.h, ih = c.ih;
     if (lo && X <= 3) {
         R t;
         if (X == 0)      t = (v[H + 1] - v[H]);
@@ -479,7 +480,7 @@ __device__ __forceinline__ R d0bw(const R *v, R h, R ih, bool c8, int X, int n, 
                               + (R)45.0 * (v[H + 1] - v[H - 1])) / (R)60.0;
         return div_const(t, h, ih);
     }
-    return d0w<R, H>(v, h, ih, c8);
+    return d0w<R, H>(v, c);
 }
 
 template <bool UNI, typename R, int H>
@@ -498,10 +499,8 @@ k_vdiv(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tmx
     const int ntx = (p.nx + VX - 1) / VX, nty = (p.ny + VY - 1) / VY;
     const int nseg = (p.nz + seg_len - 1) / seg_len;
     const long long nitems = (long long)ntx * nty * nseg;
-    const bool c8 = p.scheme_vis == 204;
     const long long N = p.N;
-    const R hh[3] = { (R)p.hx, (R)p.hy, (R)p.hz };
-    const R ihh[3] = { (R)p.inv_h[0], (R)p.inv_h[1], (R)p.inv_h[2] };
+    const D0<R> cd[3] = { D0<R>(p, 0), D0<R>(p, 1), D0<R>(p, 2) };
     if (tid == 0) {
         for (int s = 0; s < T::NZS; s++) tma::mbar_init(&zbar[s], 1);
         tma::mbar_init(&xybar[0], 1);
@@ -606,10 +605,10 @@ k_vdiv(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tmx
                             else              v[t] = zring[slot(k - H + t) * T::ZE + (m * VY + tj) * VX + ti];
                         }
                         if (!p.has_bnd) {
-                            dv[dd][m] = d0w<R, H>(v, hh[dd], ihh[dd], c8);
+                            dv[dd][m] = d0w<R, H>(v, cd[dd]);
                         } else {
                             const int X = dd == 0 ? i : (dd == 1 ? j : k), n = dd == 0 ? p.nx : (dd == 1 ? p.ny : p.nz);
-                            dv[dd][m] = d0bw<R, H>(v, hh[dd], ihh[dd], c8, X, n, p.bnd_lo[dd], p.bnd_hi[dd]);
+                            dv[dd][m] = d0bw<R, H>(v, cd[dd], X, n, p.bnd_lo[dd], p.bnd_hi[dd]);
                         }
                     }
                 }
@@ -672,7 +671,6 @@ k_vev(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tmq,
     const int ntx = (p.nx + VX - 1) / VX, nty = (p.ny + VY - 1) / VY;
     const int nseg = (p.nz + seg_len - 1) / seg_len;
     const long long nitems = (long long)ntx * nty * nseg;
-    const bool c8 = p.scheme_vis == 204;
     if (tid == 0) {
         for (int s = 0; s < T::NZS; s++) tma::mbar_init(&zbar[s], 1);
         tma::fence_mbar_init();
@@ -719,8 +717,7 @@ k_vev(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tmq,
                 R Akz = (R)metric<UNI>(p, M_AKZ, o), Aiz = (R)metric<UNI>(p, M_AIZ, o), Asz = (R)metric<UNI>(p, M_ASZ, o);
                 R Tc = at(k, 3, 0, 0);
                 R Amu = (R)p.amu_C0 * sqrt_r(Tc * Tc * Tc) / ((R)p.Tsb + Tc);      // get_Amu_kernal
-                const R ihx = (R)p.inv_h[0], ihy = (R)p.inv_h[1], ihz = (R)p.inv_h[2];
-                const R hx = (R)p.hx, hy = (R)p.hy, hz = (R)p.hz;
+                const D0<R> cx(p, 0), cy(p, 1), cz(p, 2);
                 R dk[4], di[4], ds[4];         // d/dxi, d/deta, d/dzeta of u, v, w, T
 #pragma unroll
                 for (int f = 0; f < 4; f++) {
@@ -732,13 +729,13 @@ k_vev(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tmq,
                         vz[t] = at(k - H + t, f, 0, 0);
                     }
                     if (!p.has_bnd) {
-                        dk[f] = d0w<R, H>(vx, hx, ihx, c8);
-                        di[f] = d0w<R, H>(vy, hy, ihy, c8);
-                        ds[f] = d0w<R, H>(vz, hz, ihz, c8);
+                        dk[f] = d0w<R, H>(vx, cx);
+                        di[f] = d0w<R, H>(vy, cy);
+                        ds[f] = d0w<R, H>(vz, cz);
                     } else {
-                        dk[f] = d0bw<R, H>(vx, hx, ihx, c8, i, p.nx, p.bnd_lo[0], p.bnd_hi[0]);
-                        di[f] = d0bw<R, H>(vy, hy, ihy, c8, j, p.ny, p.bnd_lo[1], p.bnd_hi[1]);
-                        ds[f] = d0bw<R, H>(vz, hz, ihz, c8, k, p.nz, p.bnd_lo[2], p.bnd_hi[2]);
+                        dk[f] = d0bw<R, H>(vx, cx, i, p.nx, p.bnd_lo[0], p.bnd_hi[0]);
+                        di[f] = d0bw<R, H>(vy, cy, j, p.ny, p.bnd_lo[1], p.bnd_hi[1]);
+                        ds[f] = d0bw<R, H>(vz, cz, k, p.nz, p.bnd_lo[2], p.bnd_hi[2]);
                     }
                 }
                 const R uk = dk[0], ui = di[0], us = ds[0], vk = dk[1], vi = di[1], vs = ds[1];
@@ -812,7 +809,7 @@ __global__ void __launch_bounds__(256) k_qcrit(Params p, double *q) {
     const long long o = lap_index(p, i + OCFD_LAP, j + OCFD_LAP, k + OCFD_LAP);
     const bool c8 = p.scheme_vis == 204;
     const double *U = p.prim[1], *V = p.prim[2], *W = p.prim[3];
-    const double ih[3] = { p.inv_h[0], p.inv_h[1], p.inv_h[2] }, hh[3] = { p.hx, p.hy, p.hz };
+    const D0<double> cd[3] = { D0<double>(p, 0), D0<double>(p, 1), D0<double>(p, 2) };
     const long long st[3] = { 1LL, p.ys, p.zs };
     const int X[3] = { i, j, k }, n[3] = { p.nx, p.ny, p.nz };
     double g[3][3];                      // g[field][direction]: uk ui us, vk vi vs, wk wi ws
@@ -821,8 +818,8 @@ __global__ void __launch_bounds__(256) k_qcrit(Params p, double *q) {
     for (int m = 0; m < 3; m++)
 #pragma unroll
         for (int d = 0; d < 3; d++)
-            g[m][d] = p.has_bnd ? d0b(F[m], o, st[d], hh[d], ih[d], c8, X[d], n[d], p.bnd_lo[d], p.bnd_hi[d])
-                                : d0(F[m], o, st[d], hh[d], ih[d], c8);
+            g[m][d] = c8 ? d0b<true>(F[m], o, st[d], cd[d], X[d], n[d], p.bnd_lo[d], p.bnd_hi[d])
+                         : d0b<false>(F[m], o, st[d], cd[d], X[d], n[d], p.bnd_lo[d], p.bnd_hi[d]);
     const double Akx = metric<UNI>(p, M_AKX, o), Aix = metric<UNI>(p, M_AIX, o), Asx = metric<UNI>(p, M_ASX, o);
     const double Aky = metric<UNI>(p, M_AKY, o), Aiy = metric<UNI>(p, M_AIY, o), Asy = metric<UNI>(p, M_ASY, o);
     const double Akz = metric<UNI>(p, M_AKZ, o), Aiz = metric<UNI>(p, M_AIZ, o), Asz = metric<UNI>(p, M_ASZ, o);
@@ -840,7 +837,8 @@ __global__ void __launch_bounds__(256) k_qcrit(Params p, double *q) {
 }
 
 // ana_time_average (src/OCFD_ana.cu:238-306): m = (n m + x) / (n + 1) for
-// d, u, v, w, T of every interior cell, n the number of samples so far
+// d, u, v, w, T of every interior cell, n the number of samples so far (each
+// operation rounded, so that a mean near zero is the formula's own)
 __global__ void k_time_average(Params p, double *mean5, int n) {
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (tid >= p.N) return;
@@ -851,7 +849,7 @@ __global__ void k_time_average(Params p, double *mean5, int n) {
 #pragma unroll
     for (int m = 0; m < 5; m++) {
         double *a = mean5 + m * p.N + tid;
-        *a = (n * *a + p.prim[m][o]) / (n + 1.);
+        *a = __dadd_rn(__dmul_rn((double)n, *a), p.prim[m][o]) / (n + 1.);
     }
 }
 
@@ -1095,22 +1093,30 @@ cudaError_t launch_ghost32(const Params &p, float *const *fields, const int *dir
 template <typename R>
 static cudaError_t launch_vis_ev_t(const Params &p, cudaStream_t st) {
     const dim3 nb((unsigned)(((p.nx + VT_X - 1) / VT_X) * ((p.ny + VT_Y - 1) / VT_Y)), (unsigned)p.nz);
-    if (p.uniform_metrics) k_vis_ev<true, R><<<nb, 256, 0, st>>>(p);
-    else                   k_vis_ev<false, R><<<nb, 256, 0, st>>>(p);
+    const bool c8 = p.scheme_vis == 204;
+    if (p.has_bnd)
+        c8 ? k_vis_ev<false, true, true, R><<<nb, 256, 0, st>>>(p) : k_vis_ev<false, true, false, R><<<nb, 256, 0, st>>>(p);
+    else if (p.uniform_metrics)
+        c8 ? k_vis_ev<true, false, true, R><<<nb, 256, 0, st>>>(p) : k_vis_ev<true, false, false, R><<<nb, 256, 0, st>>>(p);
+    else
+        c8 ? k_vis_ev<false, false, true, R><<<nb, 256, 0, st>>>(p) : k_vis_ev<false, false, false, R><<<nb, 256, 0, st>>>(p);
     return cudaGetLastError();
 }
 
-template <typename R>
+template <bool RK, typename R>
 static cudaError_t launch_vis_div_t(const Params &p, int krk, int k0, int k1, cudaStream_t st) {
     if (k1 <= k0) return cudaSuccess;
     const dim3 nb((unsigned)(((p.nx + VT_X - 1) / VT_X) * ((p.ny + VT_Y - 1) / VT_Y)), (unsigned)(k1 - k0));
-    if (krk == 0) {
-        if (p.uniform_metrics) k_vis_div<true, false, R><<<nb, 256, 0, st>>>(p, 0, k0);
-        else                   k_vis_div<false, false, R><<<nb, 256, 0, st>>>(p, 0, k0);
-    } else {
-        if (p.uniform_metrics) k_vis_div<true, true, R><<<nb, 256, 0, st>>>(p, krk, k0);
-        else                   k_vis_div<false, true, R><<<nb, 256, 0, st>>>(p, krk, k0);
-    }
+    const bool c8 = p.scheme_vis == 204;
+    if (p.has_bnd)
+        c8 ? k_vis_div<false, true, true, RK, R><<<nb, 256, 0, st>>>(p, krk, k0)
+           : k_vis_div<false, true, false, RK, R><<<nb, 256, 0, st>>>(p, krk, k0);
+    else if (p.uniform_metrics)
+        c8 ? k_vis_div<true, false, true, RK, R><<<nb, 256, 0, st>>>(p, krk, k0)
+           : k_vis_div<true, false, false, RK, R><<<nb, 256, 0, st>>>(p, krk, k0);
+    else
+        c8 ? k_vis_div<false, false, true, RK, R><<<nb, 256, 0, st>>>(p, krk, k0)
+           : k_vis_div<false, false, false, RK, R><<<nb, 256, 0, st>>>(p, krk, k0);
     return cudaGetLastError();
 }
 
@@ -1249,7 +1255,9 @@ cudaError_t launch_vis_div(const Params &p, int krk, int k0, int k1, cudaStream_
                                   : (c8 ? launch_vdiv_h<double, 4>(p, krk, st, e) : launch_vdiv_h<double, 3>(p, krk, st, e));
         if (done) return e;
     }
-    return p.mixed ? launch_vis_div_t<float>(p, krk, k0, k1, st) : launch_vis_div_t<double>(p, krk, k0, k1, st);
+    if (krk == 0)
+        return p.mixed ? launch_vis_div_t<false, float>(p, 0, k0, k1, st) : launch_vis_div_t<false, double>(p, 0, k0, k1, st);
+    return p.mixed ? launch_vis_div_t<true, float>(p, krk, k0, k1, st) : launch_vis_div_t<true, double>(p, krk, k0, k1, st);
 }
 
 // base pointers of the 12 Ev fields (FP64, or FP32 in the precision form)
