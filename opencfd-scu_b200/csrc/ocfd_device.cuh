@@ -217,75 +217,59 @@ __device__ __forceinline__ void sw_split(double tmp0, double u, double v, double
 // s[t] = f(F-3+t), t = 0..7, for both signs.
 // ---------------------------------------------------------------------------
 
-// WENO7 positive side, src/OCFD_Schemes.cu:616-663 (uses s[0..6])
-__device__ __forceinline__ double weno7_p(const double *s) {
-    double S0 = 0.0, S1 = 0.0, S2 = 0.0, S3 = 0.0, tmp, tmp1, tmp2;
-    tmp  = -2.0*s[0] +  9.0*s[1] - 18.0*s[2] + 11.0*s[3]; S0 += 960*tmp*tmp;
-    tmp1 = -6.0*s[0] + 24.0*s[1] - 30.0*s[2] + 12.0*s[3]; S0 += (1040.0)*tmp1*tmp1;
-    tmp2 = -6.0*s[0] + 18.0*( s[1] - s[2] ) + 6.0*s[3];   S0 += (1043.0)*tmp2*tmp2;
-    tmp  = tmp * tmp2; S0 += 80.0*tmp;
-    tmp  =      s[1] - 6.0*s[2] +  3.0*s[3] + 2.0*s[4]; S1 += 960*tmp*tmp;
-    tmp1 =                   6.0*s[2] - 12.0*s[3] + 6.0*s[4]; S1 += (1040.0)*tmp1*tmp1;
-    tmp2 = -6.0*s[1] + 18.0*( s[2] - s[3] ) + 6.0*s[4]; S1 += (1043.0)*tmp2*tmp2;
-    tmp  = tmp * tmp2; S1 += 80.0*tmp;
-    tmp  = -2.0*s[2] - 3.0*s[3] +  6.0*s[4] -   s[5]; S2 += 960*tmp*tmp;
-    tmp1 =                 6.0*s[3] - 12.0*s[4] + 6.0*s[5]; S2 += (1040.0)*tmp1*tmp1;
-    tmp2 = -6.0*s[2] + 18.0*(s[3] - s[4]) + 6.0*s[5]; S2 += (1043.0)*tmp2*tmp2;
-    tmp  = tmp * tmp2; S2 += 80.0*tmp;
-    tmp  = -11.0*s[3] + 18.0*s[4] -  9.0*s[5] + 2.0*s[6]; S3 += 960*tmp*tmp;
-    tmp1 =  12.0*s[3] - 30.0*s[4] + 24.0*s[5] - 6.0*s[6]; S3 += (1040.0)*tmp1*tmp1;
-    tmp2 =  -6.0*s[3] + 18.0*( s[4] -  s[5] ) + 6.0*s[6];  S3 += (1043.0)*tmp2*tmp2;
-    tmp  =  tmp * tmp2; S3 += 80.0*tmp;
-    const double e = 3.456e-4;
-    double b0 = (e + S0) * (e + S0), b1 = (e + S1) * (e + S1);
-    double b2 = (e + S2) * (e + S2), b3 = (e + S3) * (e + S3);
-    double a0 =        b1 * b2 * b3;
-    double a1 = (12.0) * b0 * b2 * b3;
-    double a2 = (18.0) * b0 * b1 * b3;
-    double a3 =  (4.0) * b0 * b1 * b2;
-    double am = a0 + a1 + a2 + a3;
-    double r = 0.0;
-    tmp = -3.0*s[0] + 13.0*s[1] - 23.0*s[2] + 25.0*s[3]; r += a0*tmp;
-    tmp =      s[1] -  5.0*s[2] + 13.0*s[3] +  3.0*s[4]; r += a1*tmp;
-    tmp =     -s[2] +  7.0*s[3] +  7.0*s[4] -      s[5]; r += a2*tmp;
-    tmp =  3.0*s[3] + 13.0*s[4] -  5.0*s[5] +      s[6]; r += a3*tmp;
-    return r / (12.0*am);
-}
+// Differences of a stencil in upwind order (P: v[t] = f(F-3+t); M:
+// f(F+4-t)): 6 first differences d[2], d[3] beside the face's cell, second
+// differences e[i] = v[i+2] - 2 v[i+1] + v[i] (i = 1 .. 3) and third ones
+// f[i] = e[i+1] - e[i].  The derivatives and candidates of the four-point
+// stencils are two or three multiply-adds of these, where each takes four of
+// the points, and cancel less.
+template <typename R> struct Diff7 {
+    R d2, d3, e1, e2, e3, f0, f1, f2, f3;
+    __device__ __forceinline__ explicit Diff7(const R *v) {
+        const R d0 = v[1] - v[0], d1 = v[2] - v[1], d4 = v[5] - v[4], d5 = v[6] - v[5];
+        d2 = v[3] - v[2]; d3 = v[4] - v[3];
+        const R e0 = d1 - d0, e4 = d5 - d4;
+        e1 = d2 - d1; e2 = d3 - d2; e3 = d4 - d3;
+        f0 = e1 - e0; f1 = e2 - e1; f2 = e3 - e2; f3 = e4 - e3;
+        d2 = (R)6.0 * d2; d3 = (R)6.0 * d3;
+    }
+    // six times the stencils' first derivatives at the face's cell, a sixth
+    // of their second ones as the smoothness indicators take them, and
+    // candidate - 12 v[3]
+    __device__ __forceinline__ R t0() const { return fma((R)2.0, f0, fma((R)3.0, e1, d2)); }
+    __device__ __forceinline__ R t1() const { return fma((R)3.0, e2, d2) - f1; }
+    __device__ __forceinline__ R t2() const { return fma((R)-3.0, e2, d3) - f2; }
+    __device__ __forceinline__ R t3() const { return fma((R)2.0, f3, fma((R)-3.0, e3, d3)); }
+    __device__ __forceinline__ R g0() const { return e1 + f0; }
+    __device__ __forceinline__ R g3() const { return e3 - f3; }
+    __device__ __forceinline__ R c0() const { return fma((R)3.0, f0, fma((R)4.0, e1, d2)); }
+    __device__ __forceinline__ R c1() const { return fma((R)4.0, e2, d2) - f1; }
+    __device__ __forceinline__ R c2() const { return fma((R)-2.0, e2, d3) - f2; }
+    __device__ __forceinline__ R c3() const { return fma((R)-2.0, e3, d3) + f3; }
+};
 
-// WENO7 negative side, src/OCFD_Schemes.cu:691-741; q[k] = s[k+1] (f(F-2..F+4))
+// WENO7 of a stencil in upwind order (uses v[0..6]), src/OCFD_Schemes.cu:616-741:
+// smoothness 960 t^2 + 1040 (6 g)^2 + 1043 (6 f)^2 + 80 t (6 f) plus its
+// epsilon.  Bound by FP64 issue; in differences about 100 FP64 operations a
+// value where the reference's point sums take 150 (64^3 Taylor-Green, five
+// steps: 2.59 -> 2.32 ms; ramp 512x128x64, two steps: 30.2 -> 28.3 ms).
+__device__ __forceinline__ double weno7_core(const double *v) {
+    const Diff7<double> q(v);
+    auto beta = [](double t, double g, double f) {
+        return fma(t, fma(960.0, t, 480.0 * f), fma(37440.0 * g, g, fma(37548.0 * f, f, 3.456e-4)));
+    };
+    double b0 = beta(q.t0(), q.g0(), q.f0), b1 = beta(q.t1(), q.e2, q.f1);
+    double b2 = beta(q.t2(), q.e3, q.f2), b3 = beta(q.t3(), q.g3(), q.f3);
+    b0 *= b0; b1 *= b1; b2 *= b2; b3 *= b3;
+    const double b01 = b0 * b1, b23 = b2 * b3;
+    const double a0 = b1 * b23, a1 = 12.0 * b0 * b23, a2 = 18.0 * b3 * b01, a3 = 4.0 * b2 * b01;
+    const double r = fma(a0, q.c0(), fma(a1, q.c1(), fma(a2, q.c2(), a3 * q.c3())));
+    return v[3] + r / (12.0 * ((a0 + a1) + (a2 + a3)));
+}
+__device__ __forceinline__ double weno7_p(const double *s) { return weno7_core(s); }
 __device__ __forceinline__ double weno7_m(const double *s8) {
-    const double *s = s8 + 1;
-    double S0 = 0.0, S1 = 0.0, S2 = 0.0, S3 = 0.0, tmp, tmp1, tmp2;
-    tmp  = -2.0*s[6] +  9.0*s[5] - 18.0*s[4] + 11.0*s[3]; S0 += 960*tmp*tmp;
-    tmp1 = -6.0*s[6] + 24.0*s[5] - 30.0*s[4] + 12.0*s[3]; S0 += (1040.0)*tmp1*tmp1;
-    tmp2 = -6.0*s[6] + 18.0*( s[5] -  s[4] ) + 6.0*s[3];  S0 += (1043.0)*tmp2*tmp2;
-    tmp  = tmp * tmp2; S0 += (80.0) * tmp;
-    tmp  =      s[5] -  6.0* s[4] + 3.0*s[3] + 2.0*s[2]; S1 += 960*tmp*tmp;
-    tmp1 =                  6.0*s[4] - 12.0* s[3] +  6.0*s[2]; S1 += (1040.0)*tmp1*tmp1;
-    tmp2 = -6.0*s[5] + 18.0*( s[4] -  s[3]) + 6.0*s[2];  S1 += (1043.0)*tmp2*tmp2;
-    tmp  = tmp *tmp2; S1 += (80.0) * tmp;
-    tmp  =    -2.0*s[4] - 3.0*s[3] + 6.0*s[2] - s[1]; S2 += 960*tmp*tmp;
-    tmp1 =                 6.0*s[3] - 12.0*s[2] + 6.0*s[1]; S2 += (1040.0)*tmp1*tmp1;
-    tmp2 = -6.0*s[4] + 18.0*(s[3] - s[2]) + 6.0*s[1]; S2 += (1043.0)*tmp2*tmp2;
-    tmp  = tmp *tmp2; S2 += (80.0) * tmp;
-    tmp  = -11.0*s[3] + 18.0*s[2] -  9.0*s[1] + 2.0*s[0]; S3 += 960*tmp*tmp;
-    tmp1 =  12.0*s[3] - 30.0*s[2] + 24.0*s[1] - 6.0*s[0]; S3 += (1040.0)*tmp1*tmp1;
-    tmp2 =  -6.0*s[3] + 18.0*( s[2] -  s[1] ) + 6.0*s[0]; S3 += (1043.0)*tmp2*tmp2;
-    tmp  =  tmp *tmp2; S3 += (80.0) * tmp;
-    const double e = 3.456e-4;
-    double b0 = (e + S0) * (e + S0), b1 = (e + S1) * (e + S1);
-    double b2 = (e + S2) * (e + S2), b3 = (e + S3) * (e + S3);
-    double a0 =        b1 * b2 * b3;
-    double a1 = (12.0) * b0 * b2 * b3;
-    double a2 = (18.0) * b0 * b1 * b3;
-    double a3 =  (4.0) * b0 * b1 * b2;
-    double am = a0 + a1 + a2 + a3;
-    double r = 0.0;
-    tmp = -3.0*s[6] + 13.0*s[5] - 23.0*s[4] + 25.0*s[3]; r += a0*tmp;
-    tmp =      s[5] -  5.0*s[4] + 13.0*s[3] +  3.0*s[2]; r += a1*tmp;
-    tmp =     -s[4] +  7.0*s[3] +  7.0*s[2] -      s[1]; r += a2*tmp;
-    tmp =  3.0*s[3] + 13.0*s[2] -  5.0*s[1] +      s[0]; r += a3*tmp;
-    return r / (12.0*am);
+    const double v[7] = { s8[7], s8[6], s8[5], s8[4], s8[3], s8[2], s8[1] };
+    return weno7_core(v);
 }
 
 // WENO5 positive side, src/OCFD_Schemes.cu:1118-1151; q = s+1 (f(F-2..F+2))
@@ -452,44 +436,35 @@ __device__ __forceinline__ double omp6_m(int flag, const double *s) {
 // stencil is mirrored; src/OCFD_Schemes.cu:391-478 (P) and :506-590 (M).
 // v[t] is the stencil in upwind order (P: f(F-3+t); M: f(F+4-t)).
 __device__ __forceinline__ double symbo_core(bool linear, const double *v) {
-    double S0, S1, S2, S3, S4, tmp;
+    // (stencils 0 .. 3 are WENO7's; the fifth, v[4..7], in the same differences)
+    const Diff7<double> q(v);
+    const double d4 = v[5] - v[4], d5 = v[6] - v[5], e4 = d5 - d4, f4 = (v[7] - v[6]) - d5 - e4;
+    double a0, a1, a2, a3, a4;
     if (linear) {
-        S0 = 0.0401954833730; S1 = 0.2493800006710; S2 = 0.4802686256260;
-        S3 = 0.2009775476730; S4 = 0.0291783426580;
+        a0 = 0.0401954833730; a1 = 0.2493800006710; a2 = 0.4802686256260;
+        a3 = 0.2009775476730; a4 = 0.0291783426580;
     } else {
-        S0 = 0.0; S1 = 0.0; S2 = 0.0; S3 = 0.0; S4 = 0.0;
-        tmp =  -2.0*v[0] +  9.0*v[1] - 18.0*v[2] + 11.0*v[3]; S0 += 720.0*tmp*tmp;
-        tmp =       v[1] -  6.0*v[2] +  3.0*v[3] +  2.0*v[4]; S1 += 720.0*tmp*tmp;
-        tmp =  -2.0*v[2] -  3.0*v[3] +  6.0*v[4] -      v[5]; S2 += 720.0*tmp*tmp;
-        tmp = -11.0*v[3] + 18.0*v[4] -  9.0*v[5] +  2.0*v[6]; S3 += 720.0*tmp*tmp;
-        tmp = -26.0*v[4] + 57.0*v[5] - 42.0*v[6] + 11.0*v[7]; S4 += 720.0*tmp*tmp;
-        tmp = -6.0*v[0] + 24.0*v[1] - 30.0*v[2] + 12.0*v[3]; S0 += 780.0*tmp*tmp;
-        tmp =                    6.0*v[2] - 12.0*v[3] +  6.0*v[4]; S1 += 780.0*tmp*tmp;
-        tmp =                    6.0*v[3] - 12.0*v[4] +  6.0*v[5]; S2 += 780.0*tmp*tmp;
-        tmp = 12.0*v[3] - 30.0*v[4] + 24.0*v[5] -  6.0*v[6]; S3 += 780.0*tmp*tmp;
-        tmp = 18.0*v[4] - 48.0*v[5] + 42.0*v[6] - 12.0*v[7]; S4 += 780.0*tmp*tmp;
-        tmp = -6.0*v[0] + 18.0*( v[1] - v[2] ) + 6.0*v[3]; S0 += 781.0*tmp*tmp;
-        tmp = -6.0*v[1] + 18.0*( v[2] - v[3] ) + 6.0*v[4]; S1 += 781.0*tmp*tmp;
-        tmp = -6.0*v[2] + 18.0*( v[3] - v[4] ) + 6.0*v[5]; S2 += 781.0*tmp*tmp;
-        tmp = -6.0*v[3] + 18.0*( v[4] - v[5] ) + 6.0*v[6]; S3 += 781.0*tmp*tmp;
-        tmp = -6.0*v[4] + 18.0*( v[5] - v[6] ) + 6.0*v[7]; S4 += 781.0*tmp*tmp;
+        auto beta = [](double t, double g, double f) {
+            return fma(720.0 * t, t, fma(28080.0 * g, g, 28116.0 * f * f));
+        };
+        const double S0 = beta(q.t0(), q.g0(), q.f0), S1 = beta(q.t1(), q.e2, q.f1);
+        const double S2 = beta(q.t2(), q.e3, q.f2), S3 = beta(q.t3(), q.g3(), q.f3);
+        double S4 = beta(fma(11.0, f4, fma(-9.0, e4, 6.0 * d4)), fma(-2.0, f4, e4), f4);
         S4 = fmax(fmax(fmax(S0, S1), fmax(S2, S3)), S4);
         const double e = 2.592e-6;
-        double t0 =  (0.0401954833730)*(e+S1)*(e+S2)*(e+S3)*(e+S4);
-        double t1 =  (0.2493800006710)*(e+S0)*(e+S2)*(e+S3)*(e+S4);
-        double t2 =  (0.4802686256260)*(e+S0)*(e+S1)*(e+S3)*(e+S4);
-        double t3 =  (0.2009775476730)*(e+S0)*(e+S1)*(e+S2)*(e+S4);
-        S4 =         (0.0291783426580)*(e+S0)*(e+S1)*(e+S2)*(e+S3);
-        S3 = t3; S2 = t2; S1 = t1; S0 = t0;
+        const double b0 = e + S0, b1 = e + S1, b2 = e + S2, b3 = e + S3, b4 = e + S4;
+        const double b01 = b0 * b1, b23 = b2 * b3, b014 = b01 * b4, b234 = b23 * b4;
+        a0 = 0.0401954833730 * b1 * b234;
+        a1 = 0.2493800006710 * b0 * b234;
+        a2 = 0.4802686256260 * b3 * b014;
+        a3 = 0.2009775476730 * b2 * b014;
+        a4 = 0.0291783426580 * b01 * b23;
     }
-    double am = S0 + S1 + S2 + S3 + S4;
-    double r = 0.0;
-    tmp = -3.0*v[0] + 13.0*v[1] - 23.0*v[2] + 25.0*v[3]; r += S0*tmp;
-    tmp =      v[1] -  5.0*v[2] + 13.0*v[3] +  3.0*v[4]; r += S1*tmp;
-    tmp =     -v[2] +  7.0*v[3] +  7.0*v[4] -      v[5]; r += S2*tmp;
-    tmp =  3.0*v[3] + 13.0*v[4] -  5.0*v[5] +      v[6]; r += S3*tmp;
-    tmp = 25.0*v[4] - 23.0*v[5] + 13.0*v[6] -  3.0*v[7]; r += S4*tmp;
-    return r / (12.0*am);
+    const double am = ((a0 + a1) + (a2 + a3)) + a4;
+    // candidate 4: 12 v[4] - 6 d4 + 4 e4 - 3 f4 = 12 v[3] + 6 d3 - 6 e3 + 4 e4 - 3 f4
+    const double c4 = fma(-3.0, f4, fma(4.0, e4, fma(-6.0, q.e3, q.d3)));
+    const double r = fma(a0, q.c0(), fma(a1, q.c1(), fma(a2, q.c2(), fma(a3, q.c3(), a4 * c4))));
+    return v[3] + r / (12.0 * am);
 }
 
 __device__ __forceinline__ double symbo_p(int lmt, double tv_lim, double tv_max, const double *s) {

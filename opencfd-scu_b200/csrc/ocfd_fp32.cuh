@@ -114,60 +114,24 @@ __device__ __forceinline__ float up7_m_q(const float *s) {
                      - 38.0f*s[2] + 4.0f*s[1], 420.0f, 1.0f / 420.0f);
 }
 
-// WENO7 smoothness indicator of the 4-point sub-stencil q[0..3] written as
-// in the reference (the 960 / 1040 / 1043 / 80 form, first/second/third
-// differences t, t1, t2), for sub-stencil index k
-__device__ __forceinline__ float w7_beta(float t, float t1, float t2) {
-    return 960.0f*t*t + 1040.0f*t1*t1 + 1043.0f*t2*t2 + 80.0f*(t*t2);
+// WENO7 of a stencil in upwind order (v[0..6]), as the FP64 form's differences;
+// the weights one quotient each, where a common denominator would overflow
+__device__ __forceinline__ float weno7_core(const float *v) {
+    const Diff7<float> q(v);
+    auto beta = [](float t, float g, float f) {
+        return fmaf(t, fmaf(960.0f, t, 480.0f * f), fmaf(37440.0f * g, g, fmaf(37548.0f * f, f, 3.456e-4f)));
+    };
+    const float b0 = beta(q.t0(), q.g0(), q.f0), b1 = beta(q.t1(), q.e2, q.f1);
+    const float b2 = beta(q.t2(), q.e3, q.f2), b3 = beta(q.t3(), q.g3(), q.f3);
+    const float a0 = fdiv(1.0f, b0 * b0), a1 = fdiv(12.0f, b1 * b1);
+    const float a2 = fdiv(18.0f, b2 * b2), a3 = fdiv(4.0f, b3 * b3);
+    const float r = fmaf(a0, q.c0(), fmaf(a1, q.c1(), fmaf(a2, q.c2(), a3 * q.c3())));
+    return v[3] + fdiv(r, 12.0f * ((a0 + a1) + (a2 + a3)));
 }
-
-// WENO7, s[0..6] = f(F-3..F+3) (positive side)
-__device__ __forceinline__ float weno7_p(const float *s) {
-    const float S0 = w7_beta(-2.0f*s[0] + 9.0f*s[1] - 18.0f*s[2] + 11.0f*s[3],
-                             -6.0f*s[0] + 24.0f*s[1] - 30.0f*s[2] + 12.0f*s[3],
-                             -6.0f*s[0] + 18.0f*(s[1] - s[2]) + 6.0f*s[3]);
-    const float S1 = w7_beta(s[1] - 6.0f*s[2] + 3.0f*s[3] + 2.0f*s[4],
-                             6.0f*s[2] - 12.0f*s[3] + 6.0f*s[4],
-                             -6.0f*s[1] + 18.0f*(s[2] - s[3]) + 6.0f*s[4]);
-    const float S2 = w7_beta(-2.0f*s[2] - 3.0f*s[3] + 6.0f*s[4] - s[5],
-                             6.0f*s[3] - 12.0f*s[4] + 6.0f*s[5],
-                             -6.0f*s[2] + 18.0f*(s[3] - s[4]) + 6.0f*s[5]);
-    const float S3 = w7_beta(-11.0f*s[3] + 18.0f*s[4] - 9.0f*s[5] + 2.0f*s[6],
-                             12.0f*s[3] - 30.0f*s[4] + 24.0f*s[5] - 6.0f*s[6],
-                             -6.0f*s[3] + 18.0f*(s[4] - s[5]) + 6.0f*s[6]);
-    const float e = 3.456e-4f;
-    const float a0 = fdiv(1.0f, (e + S0) * (e + S0)), a1 = fdiv(12.0f, (e + S1) * (e + S1));
-    const float a2 = fdiv(18.0f, (e + S2) * (e + S2)), a3 = fdiv(4.0f, (e + S3) * (e + S3));
-    const float r = a0 * (-3.0f*s[0] + 13.0f*s[1] - 23.0f*s[2] + 25.0f*s[3])
-                  + a1 * (s[1] - 5.0f*s[2] + 13.0f*s[3] + 3.0f*s[4])
-                  + a2 * (-s[2] + 7.0f*s[3] + 7.0f*s[4] - s[5])
-                  + a3 * (3.0f*s[3] + 13.0f*s[4] - 5.0f*s[5] + s[6]);
-    return fdiv(r, 12.0f * (a0 + a1 + a2 + a3));
-}
-
-// WENO7 negative side, s8[1..7] = f(F-2..F+4)
+__device__ __forceinline__ float weno7_p(const float *s) { return weno7_core(s); }
 __device__ __forceinline__ float weno7_m(const float *s8) {
-    const float *s = s8 + 1;
-    const float S0 = w7_beta(-2.0f*s[6] + 9.0f*s[5] - 18.0f*s[4] + 11.0f*s[3],
-                             -6.0f*s[6] + 24.0f*s[5] - 30.0f*s[4] + 12.0f*s[3],
-                             -6.0f*s[6] + 18.0f*(s[5] - s[4]) + 6.0f*s[3]);
-    const float S1 = w7_beta(s[5] - 6.0f*s[4] + 3.0f*s[3] + 2.0f*s[2],
-                             6.0f*s[4] - 12.0f*s[3] + 6.0f*s[2],
-                             -6.0f*s[5] + 18.0f*(s[4] - s[3]) + 6.0f*s[2]);
-    const float S2 = w7_beta(-2.0f*s[4] - 3.0f*s[3] + 6.0f*s[2] - s[1],
-                             6.0f*s[3] - 12.0f*s[2] + 6.0f*s[1],
-                             -6.0f*s[4] + 18.0f*(s[3] - s[2]) + 6.0f*s[1]);
-    const float S3 = w7_beta(-11.0f*s[3] + 18.0f*s[2] - 9.0f*s[1] + 2.0f*s[0],
-                             12.0f*s[3] - 30.0f*s[2] + 24.0f*s[1] - 6.0f*s[0],
-                             -6.0f*s[3] + 18.0f*(s[2] - s[1]) + 6.0f*s[0]);
-    const float e = 3.456e-4f;
-    const float a0 = fdiv(1.0f, (e + S0) * (e + S0)), a1 = fdiv(12.0f, (e + S1) * (e + S1));
-    const float a2 = fdiv(18.0f, (e + S2) * (e + S2)), a3 = fdiv(4.0f, (e + S3) * (e + S3));
-    const float r = a0 * (-3.0f*s[6] + 13.0f*s[5] - 23.0f*s[4] + 25.0f*s[3])
-                  + a1 * (s[5] - 5.0f*s[4] + 13.0f*s[3] + 3.0f*s[2])
-                  + a2 * (-s[4] + 7.0f*s[3] + 7.0f*s[2] - s[1])
-                  + a3 * (3.0f*s[3] + 13.0f*s[2] - 5.0f*s[1] + s[0]);
-    return fdiv(r, 12.0f * (a0 + a1 + a2 + a3));
+    const float v[7] = { s8[7], s8[6], s8[5], s8[4], s8[3], s8[2], s8[1] };
+    return weno7_core(v);
 }
 
 // WENO5 (positive side uses s8[1..5], negative side s8[2..6])
