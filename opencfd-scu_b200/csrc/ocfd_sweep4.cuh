@@ -33,8 +33,13 @@ enum { K_HYBC = 0, K_W7 = 1 };
 // ring value sv of point Q of line col
 template <int RING, int LC, typename R>
 __device__ __forceinline__ R rv(const R *ring, int col, int sv, int Q) {
-    return ring[(sv * RING + (Q & (RING - 1))) * LC + col];
+    return ring[(sv * RING + ring_slot<RING>(Q)) * LC + col];
 }
+
+// lines, and points of the ring, a warp: a pass's window of LY + 7 points
+// fits the ring exactly enough for five blocks of the y and z walks an SM
+template <int DIR> struct Shape4 { static constexpr int LC = 8, RING = 12; };
+template <> struct Shape4<0> { static constexpr int LC = 1, RING = 64; };
 
 // One sign of a characteristic face F+1/2: the sign's 7-point stencil of
 // the five split fields, projected on each characteristic field, the
@@ -215,18 +220,16 @@ __device__ __forceinline__ void du_rule_cell(const Params &p, const R *ring, int
 // MINB: resident blocks per SM the register budget is fitted to; 3 (168
 // registers, a few spills) runs faster than 2 (no spills) on the
 // characteristic faces.
-// The walk: a warp covers LC lines and LY = 32 / LC consecutive cells of
-// each, LY cells per pass.  Per pass every lane splits one new point into
-// the ring, forms the flux of the face on the right of its cell into the
-// face buffer (FR = 2 LY slots per line, so a pass never overwrites a face
-// that the previous pass's lanes still read), then adds its cell's du with
-// the face on its left from the buffer.
+// The walk: a warp covers LC lines and LY = 32 / LC consecutive faces of
+// each per pass, from the one left of the segment's first cell on.  Per pass
+// every lane splits one new point into the ring, forms its face's flux into
+// the face buffer (slot 0 of a line keeps the previous pass's last face), then
+// adds the du of the cell on the face's left, with the face on that cell's
+// left from the buffer.
 template <int DIR, bool UNI, bool EPS0, int KIND, int MINB, bool SPLIT, typename R>
 __global__ void __launch_bounds__(32 * SW, MINB) k_sweep4(const __grid_constant__ Params p, int seg_len) {
-    constexpr int LC = Shape<DIR>::LC, LY = 32 / LC, RING = Shape<DIR>::RING, FR = 2 * LY;
-    // the next pass's points overwrite slots this pass reads unless the
-    // ring spans both windows
-    constexpr bool SYNC2 = 2 * LY + 6 >= RING;
+    constexpr int LC = Shape4<DIR>::LC, LY = 32 / LC, RING = Shape4<DIR>::RING, FR = LY + 1;
+    static_assert(LY + 7 <= RING, "a pass's window fits the ring");
     extern __shared__ __align__(16) unsigned char smem4[];   // per warp: ring, then face buffer
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int col = lane % LC, ly = lane / LC;
@@ -270,8 +273,8 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep4(const __grid_constant_
     const bool lo = p.bnd_lo[DIR], hi = p.bnd_hi[DIR];
     const R h = (R)(DIR == 0 ? p.hx : (DIR == 1 ? p.hy : p.hz)), ih = (R)p.inv_h[DIR];
 
-    // points y0-4 .. y0+3 and the face left of cell y0
-    for (int r = ly; r < 8; r += LY) {
+    // points y0-4 .. y0+2
+    for (int r = ly; r < 7; r += LY) {
         if (colok) {
             R q5[5];
             const long long o = base + (long long)(y0 - 4 + r) * sd;
@@ -279,16 +282,8 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep4(const __grid_constant_
             ring_put<DIR, RING, LC, UNI, EPS0>(p, ring, col, y0 - 4 + r, o, q5);
         }
     }
-    __syncwarp();
-    if (ly == 0 && colok) {
-        const int hf = KIND == K_HYBC ? flag_at(p, DIR, fl, (long long)y0 * fst) : 2;
-        R cur[10];
-        face4<KIND, RING, LC, UNI, SPLIT>(p, DIR, ring, col, y0 - 1, n, hf, base + (long long)(y0 - 1) * sd, sd, lo, hi, cur);
-#pragma unroll
-        for (int sv = 0; sv < 10; sv++) fbuf[(sv * FR + ((y0 - 1) & (FR - 1))) * LC + col] = cur[sv];
-    }
 
-    for (int Y0 = y0; Y0 < y1; Y0 += LY) {
+    for (int Y0 = y0 - 1; Y0 < y1; Y0 += LY) {
         const int P = Y0 + 4 + ly;
         const int F = Y0 + ly;
         const bool valid = colok && F < y1;
@@ -304,13 +299,13 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep4(const __grid_constant_
         if (valid) {
             face4<KIND, RING, LC, UNI, SPLIT>(p, DIR, ring, col, F, n, hflag, base + (long long)F * sd, sd, lo, hi, cur);
 #pragma unroll
-            for (int sv = 0; sv < 10; sv++) fbuf[(sv * FR + (F & (FR - 1))) * LC + col] = cur[sv];
+            for (int sv = 0; sv < 10; sv++) fbuf[(sv * FR + ly + 1) * LC + col] = cur[sv];
         }
         __syncwarp();
-        if (valid) {
+        if (valid && F >= y0) {
             R prv[10];
 #pragma unroll
-            for (int sv = 0; sv < 10; sv++) prv[sv] = fbuf[(sv * FR + ((F - 1) & (FR - 1))) * LC + col];
+            for (int sv = 0; sv < 10; sv++) prv[sv] = fbuf[(sv * FR + ly) * LC + col];
             const long long ci = OCFD_IDX(p, cb + (long long)F * cst, N);
             const R aj = (R)metric<UNI>(p, M_AJAC, base + (long long)F * sd);
             if (p.has_bnd && rule_cell(p, DIR, F, n)) {
@@ -325,7 +320,12 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep4(const __grid_constant_
                 else          add_du<false>(du, N, ci, aj, h, ih, cur, prv, old);
             }
         }
-        if (SYNC2) __syncwarp();
+        // the next pass overwrites points and faces this one has read
+        __syncwarp();
+        if (valid && ly == LY - 1) {
+#pragma unroll
+            for (int sv = 0; sv < 10; sv++) fbuf[sv * FR * LC + col] = cur[sv];
+        }
     }
 }
 
@@ -474,22 +474,13 @@ __global__ void __launch_bounds__(32 * FIX4W) k_sweep4_fix(const __grid_constant
 
 template <int DIR, bool UNI, bool EPS0, int KIND, int MINB, bool SPLIT, typename R>
 cudaError_t launch_dir4(const Params &p, cudaStream_t st) {
-    constexpr int LC = Shape<DIR>::LC, LY = 32 / LC;
+    constexpr int LC = Shape4<DIR>::LC, LY = 32 / LC;
     const int n = DIR == 0 ? p.nx : (DIR == 1 ? p.ny : p.nz);
     const long long ngx = (p.nx + LC - 1) / LC;
     const long long groups = DIR == 0 ? (long long)p.ny * p.nz : ngx * (DIR == 1 ? p.nz : p.ny);
-    // split lines into segments when there are fewer than about four waves
-    // of warps; a segment re-splits 8 points and re-forms one face
-    const long long want = 4LL * 148 * MINB * SW;
-    long long nseg = (want + groups - 1) / groups;
-    long long maxseg = n / (4 * LY) > 0 ? n / (4 * LY) : 1;
-    if (nseg > maxseg) nseg = maxseg;
-    if (nseg < 1) nseg = 1;
-    int seg_len = (int)((n + nseg - 1) / nseg);
-    seg_len = (seg_len + LY - 1) / LY * LY;
-    nseg = (n + seg_len - 1) / seg_len;
-    dim3 grid((unsigned)((groups + SW - 1) / SW), (unsigned)nseg);
-    constexpr int smem = SW * 10 * (Shape<DIR>::RING + 2 * LY) * LC * (int)sizeof(R);
+    const int seg_len = segment_cells(groups, n, LY, 148LL * MINB * SW, 3);
+    dim3 grid((unsigned)((groups + SW - 1) / SW), (unsigned)((n + seg_len - 1) / seg_len));
+    constexpr int smem = SW * 10 * (Shape4<DIR>::RING + LY + 1) * LC * (int)sizeof(R);
     static bool attr_set = false;             // above the 48 KB default
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(k_sweep4<DIR, UNI, EPS0, KIND, MINB, SPLIT, R>,
@@ -501,10 +492,11 @@ cudaError_t launch_dir4(const Params &p, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// FP64: register budget for 3 blocks per SM; FP32 (the precision form): 4
+// FP64: register budget for 3 blocks per SM (characteristic faces), 5 (WENO7);
+// FP32 (the precision form): 4, 5
 template <bool UNI, bool EPS0, int KIND, bool SPLIT, typename R>
 cudaError_t dir4s(const Params &p, int dir, cudaStream_t st) {
-    constexpr int MINB = sizeof(R) == 8 ? 3 : 4;
+    constexpr int MINB = KIND == K_W7 ? 5 : sizeof(R) == 8 ? 3 : 4;
     if (dir == 0) return launch_dir4<0, UNI, EPS0, KIND, MINB, SPLIT, R>(p, st);
     if (dir == 1) return launch_dir4<1, UNI, EPS0, KIND, MINB, SPLIT, R>(p, st);
     return launch_dir4<2, UNI, EPS0, KIND, MINB, SPLIT, R>(p, st);
