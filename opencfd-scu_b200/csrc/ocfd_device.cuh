@@ -500,12 +500,13 @@ __device__ __forceinline__ double symbo_m(int lmt, double tv_lim, double tv_max,
 }
 
 // CD6 / CD8 first difference, 60 h or 840 h times the derivative, src/OCFD_Schemes.cu:96-126
+// (multiply-adds spelled out, so that every kernel forms the same bits)
 __device__ __forceinline__ double cd6(double sm3, double sm2, double sm1, double sp1, double sp2, double sp3) {
-    return 45.0*(sp1 - sm1) - 9.0*(sp2 - sm2) + (sp3 - sm3);
+    return fma(45.0, sp1 - sm1, fma(-9.0, sp2 - sm2, sp3 - sm3));
 }
 __device__ __forceinline__ double cd8(double sm4, double sm3, double sm2, double sm1,
                                       double sp1, double sp2, double sp3, double sp4) {
-    return 672.0*(sp1 - sm1) - 168.0*(sp2 - sm2) + 32.0*(sp3 - sm3) - 3.0*(sp4 - sm4);
+    return fma(672.0, sp1 - sm1, fma(-168.0, sp2 - sm2, fma(32.0, sp3 - sm3, -3.0*(sp4 - sm4))));
 }
 
 // ---------------------------------------------------------------------------

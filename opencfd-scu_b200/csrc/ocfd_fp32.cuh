@@ -338,11 +338,11 @@ __device__ __forceinline__ float dot5(const float S[5], float x0, float x1, floa
 
 // CD6 / CD8 first derivative
 __device__ __forceinline__ float cd6(float sm3, float sm2, float sm1, float sp1, float sp2, float sp3) {
-    return 45.0f*(sp1 - sm1) - 9.0f*(sp2 - sm2) + (sp3 - sm3);
+    return fmaf(45.0f, sp1 - sm1, fmaf(-9.0f, sp2 - sm2, sp3 - sm3));
 }
 __device__ __forceinline__ float cd8(float sm4, float sm3, float sm2, float sm1,
                                      float sp1, float sp2, float sp3, float sp4) {
-    return 672.0f*(sp1 - sm1) - 168.0f*(sp2 - sm2) + 32.0f*(sp3 - sm3) - 3.0f*(sp4 - sm4);
+    return fmaf(672.0f, sp1 - sm1, fmaf(-168.0f, sp2 - sm2, fmaf(32.0f, sp3 - sm3, -3.0f*(sp4 - sm4))));
 }
 
 }  // namespace ocfd

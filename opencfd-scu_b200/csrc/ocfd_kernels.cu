@@ -198,9 +198,8 @@ __device__ __forceinline__ R d0b(const R *f, long long o, long long s, const D0<
         R t;
         if (X == 0)      t = (f[o + s] - f[o]);
         else if (X == 1) t = (f[o + s] - f[o - s]) * (R)0.5;
-        else if (X == 2) t = (f[o - 2 * s] - (R)8.0 * f[o - s] + (R)8.0 * f[o + s] - f[o + 2 * s]) / (R)12.0;
-        else             t = (f[o + 3 * s] - f[o - 3 * s] - (R)9.0 * (f[o + 2 * s] - f[o - 2 * s])
-                             + (R)45.0 * (f[o + s] - f[o - s])) / (R)60.0;
+        else if (X == 2) t = fma((R)8.0, f[o + s] - f[o - s], f[o - 2 * s] - f[o + 2 * s]) / (R)12.0;
+        else             t = fma((R)45.0, f[o + s] - f[o - s], fma((R)-9.0, f[o + 2 * s] - f[o - 2 * s], f[o + 3 * s] - f[o - 3 * s])) / (R)60.0;
         return div_const(t, h, ih);
     }
     if (hi && X >= n - 4) {
@@ -208,9 +207,8 @@ __device__ __forceinline__ R d0b(const R *f, long long o, long long s, const D0<
         const int q = X - n;
         if (q == -1)      t = (f[o] - f[o - s]);
         else if (q == -2) t = (f[o + s] - f[o - s]) * (R)0.5;
-        else if (q == -3) t = (f[o - 2 * s] - (R)8.0 * f[o - s] + (R)8.0 * f[o + s] - f[o + 2 * s]) / (R)12.0;
-        else              t = (f[o + 3 * s] - f[o - 3 * s] - (R)9.0 * (f[o + 2 * s] - f[o - 2 * s])
-                              + (R)45.0 * (f[o + s] - f[o - s])) / (R)60.0;
+        else if (q == -3) t = fma((R)8.0, f[o + s] - f[o - s], f[o - 2 * s] - f[o + 2 * s]) / (R)12.0;
+        else              t = fma((R)45.0, f[o + s] - f[o - s], fma((R)-9.0, f[o + 2 * s] - f[o - 2 * s], f[o + 3 * s] - f[o - 3 * s])) / (R)60.0;
         return div_const(t, h, ih);
     }
     return d0<C8>(f, o, s, c);
@@ -243,6 +241,38 @@ __device__ __forceinline__ bool tile_cell(const Params &p, int &i, int &j, int &
     return true;
 }
 
+// Stress, heat flux and the 12 Ev of one cell from its derivatives along the
+// grid directions (uk, ui, us ...) and its metrics m, of k_vis_ev and k_vev.
+// The multiply-adds are spelled out: the two form the same bits.
+template <bool UNI, typename R>
+__device__ __forceinline__ void vis_fluxes(const Params &p, long long o, const R (&m)[3][3], R Amu,
+                                           R uk, R ui, R us, R vk, R vi, R vs, R wk, R wi, R ws, R Tk, R Ti, R Ts,
+                                           R uu, R vv, R ww) {
+    auto dot = [](const R (&a)[3], R x, R y, R z) { return fma(a[0], x, fma(a[1], y, a[2] * z)); };
+    auto grad = [&](R k_, R i_, R s_, int c) { return fma(k_, m[0][c], fma(i_, m[1][c], s_ * m[2][c])); };
+    const R ux = grad(uk, ui, us, 0), vx = grad(vk, vi, vs, 0), wx = grad(wk, wi, ws, 0);
+    const R uy = grad(uk, ui, us, 1), vy = grad(vk, vi, vs, 1), wy = grad(wk, wi, ws, 1);
+    const R uz = grad(uk, ui, us, 2), vz = grad(vk, vi, vs, 2), wz = grad(wk, wi, ws, 2);
+    const R d23 = (R)(-2.0 / 3.0) * (ux + vy + wz);
+    const R s11 = fma((R)2.0, ux, d23) * Amu, s22 = fma((R)2.0, vy, d23) * Amu, s33 = fma((R)2.0, wz, d23) * Amu;
+    const R s12 = (uy + vx) * Amu, s13 = (uz + wx) * Amu, s23 = (vz + wy) * Amu;
+    const R Amuk = Amu * (R)p.vis_c;
+    const R vel[3] = { uu, vv, ww };
+    const R E1 = fma(Amuk, grad(Tk, Ti, Ts, 0), dot(vel, s11, s12, s13));
+    const R E2 = fma(Amuk, grad(Tk, Ti, Ts, 1), dot(vel, s12, s22, s23));
+    const R E3 = fma(Amuk, grad(Tk, Ti, Ts, 2), dot(vel, s13, s23, s33));
+    const R Aj1 = (R)metric<UNI>(p, M_AJAC, o);
+    R *const evb = ev_r<R>(p);
+#pragma unroll
+    for (int dd = 0; dd < 3; dd++) {
+        const R a[3] = { m[dd][0] * Aj1, m[dd][1] * Aj1, m[dd][2] * Aj1 };
+        R *ev = evb + (long long)(4 * dd) * p.lapN + o;
+        const R v[4] = { dot(a, s11, s12, s13), dot(a, s12, s22, s23), dot(a, s13, s23, s33), dot(a, E1, E2, E3) };
+#pragma unroll
+        for (int q = 0; q < 4; q++) ev[q * p.lapN] = v[q];
+    }
+}
+
 // Ev1..4 of all three directions (vis_flux_ker :178-236).  The 12 velocity
 // and temperature derivatives (du_viscous_Jacobian3d_init :58-77) are formed
 // here from the LAP-box primitives instead of being stored; the stress and
@@ -257,9 +287,9 @@ __global__ void __launch_bounds__(256, sizeof(R) == 8 ? 4 : 6) k_vis_ev(const __
     long long tid;
     if (!tile_cell(p, i, j, k, tid)) return;
     long long o = lap_index(p, i + OCFD_LAP, j + OCFD_LAP, k + OCFD_LAP);
-    R Akx = (R)metric<UNI>(p, M_AKX, o), Aix = (R)metric<UNI>(p, M_AIX, o), Asx = (R)metric<UNI>(p, M_ASX, o);
-    R Aky = (R)metric<UNI>(p, M_AKY, o), Aiy = (R)metric<UNI>(p, M_AIY, o), Asy = (R)metric<UNI>(p, M_ASY, o);
-    R Akz = (R)metric<UNI>(p, M_AKZ, o), Aiz = (R)metric<UNI>(p, M_AIZ, o), Asz = (R)metric<UNI>(p, M_ASZ, o);
+    R m[3][3];                            // [direction][component]
+#pragma unroll
+    for (int q = 0; q < 9; q++) m[q / 3][q % 3] = (R)metric<UNI>(p, M_AKX + q, o);
     const R *U = prim_r<R>(p, 1), *V = prim_r<R>(p, 2), *W = prim_r<R>(p, 3), *TT = prim_r<R>(p, 4);
     R Tc = TT[o];
     R Amu = (R)p.amu_C0 * sqrt_r(Tc * Tc * Tc) / ((R)p.Tsb + Tc);      // get_Amu_kernal
@@ -269,43 +299,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 8 ? 4 : 6) k_vis_ev(const __
     auto dz = [&](const R *f) { return BND ? d0b<C8>(f, o, p.zs, cz, k, p.nz, p.bnd_lo[2], p.bnd_hi[2]) : d0<C8>(f, o, p.zs, cz); };
     const R uk = dx(U), ui = dy(U), us = dz(U), vk = dx(V), vi = dy(V), vs = dz(V);
     const R wk = dx(W), wi = dy(W), ws = dz(W), Tk = dx(TT), Ti = dy(TT), Ts = dz(TT);
-    R ux = uk*Akx + ui*Aix + us*Asx;
-    R vx = vk*Akx + vi*Aix + vs*Asx;
-    R wx = wk*Akx + wi*Aix + ws*Asx;
-    R uy = uk*Aky + ui*Aiy + us*Asy;
-    R vy = vk*Aky + vi*Aiy + vs*Asy;
-    R wy = wk*Aky + wi*Aiy + ws*Asy;
-    R uz = uk*Akz + ui*Aiz + us*Asz;
-    R vz = vk*Akz + vi*Aiz + vs*Asz;
-    R wz = wk*Akz + wi*Aiz + ws*Asz;
-    R div = ux + vy + wz;
-    R s11 = ((R)2.0*ux - (R)(2.0/3.0)*div) * Amu;
-    R s22 = ((R)2.0*vy - (R)(2.0/3.0)*div) * Amu;
-    R s33 = ((R)2.0*wz - (R)(2.0/3.0)*div) * Amu;
-    R s12 = (uy + vx) * Amu;
-    R s13 = (uz + wx) * Amu;
-    R s23 = (vz + wy) * Amu;
-    R uu = U[o], vv = V[o], ww = W[o];
-    R Amuk = Amu * (R)p.vis_c;
-    R Tx = Tk*Akx + Ti*Aix + Ts*Asx;
-    R Ty = Tk*Aky + Ti*Aiy + Ts*Asy;
-    R Tz = Tk*Akz + Ti*Aiz + Ts*Asz;
-    R E1 = uu*s11 + vv*s12 + ww*s13 + Amuk*Tx;
-    R E2 = uu*s12 + vv*s22 + ww*s23 + Amuk*Ty;
-    R E3 = uu*s13 + vv*s23 + ww*s33 + Amuk*Tz;
-    R Aj1 = (R)metric<UNI>(p, M_AJAC, o);
-    R *const evb = ev_r<R>(p);
-#pragma unroll
-    for (int dd = 0; dd < 3; dd++) {
-        R akx = (R)metric<UNI>(p, M_AKX + 3 * dd, o) * Aj1;
-        R aky = (R)metric<UNI>(p, M_AKX + 3 * dd + 1, o) * Aj1;
-        R akz = (R)metric<UNI>(p, M_AKX + 3 * dd + 2, o) * Aj1;
-        R *ev = evb + (long long)(4 * dd) * p.lapN;
-        ev[o]              = (akx*s11 + aky*s12 + akz*s13);
-        ev[p.lapN + o]     = (akx*s12 + aky*s22 + akz*s23);
-        ev[2 * p.lapN + o] = (akx*s13 + aky*s23 + akz*s33);
-        ev[3 * p.lapN + o] = (akx*E1  + aky*E2  + akz*E3);
-    }
+    vis_fluxes<UNI, R>(p, o, m, Amu, uk, ui, us, vk, vi, vs, wk, wi, ws, Tk, Ti, Ts, U[o], V[o], W[o]);
 }
 
 // RK stage (src/OCFD_time.cu:44-94) + cons_to_pri (src/commen_kernel.cu:77-109)
@@ -409,10 +403,10 @@ __global__ void __launch_bounds__(256, BND || sizeof(R) == 4 ? 6 : 3) k_vis_div(
         for (int m = 0; m < 4; m++) {
             const R *f = evb + (long long)(4 * dd + m) * p.lapN;
             if (!BND) {
-                acc[m + 1] += ajac * d0<C8>(f, o, st[dd], D0<R>(p, dd));
+                acc[m + 1] = fma(ajac, d0<C8>(f, o, st[dd], D0<R>(p, dd)), acc[m + 1]);
             } else {
                 const int X = dd == 0 ? i : (dd == 1 ? j : k), n = dd == 0 ? p.nx : (dd == 1 ? p.ny : p.nz);
-                acc[m + 1] += ajac * d0b<C8>(f, o, st[dd], D0<R>(p, dd), X, n, p.bnd_lo[dd], p.bnd_hi[dd]);
+                acc[m + 1] = fma(ajac, d0b<C8>(f, o, st[dd], D0<R>(p, dd), X, n, p.bnd_lo[dd], p.bnd_hi[dd]), acc[m + 1]);
             }
         }
     }
@@ -465,9 +459,8 @@ __device__ __forceinline__ R d0bw(const R *v, const D0<R> &c, int X, int n, bool
         R t;
         if (X == 0)      t = (v[H + 1] - v[H]);
         else if (X == 1) t = (v[H + 1] - v[H - 1]) * (R)0.5;
-        else if (X == 2) t = (v[H - 2] - (R)8.0 * v[H - 1] + (R)8.0 * v[H + 1] - v[H + 2]) / (R)12.0;
-        else             t = (v[H + 3] - v[H - 3] - (R)9.0 * (v[H + 2] - v[H - 2])
-                             + (R)45.0 * (v[H + 1] - v[H - 1])) / (R)60.0;
+        else if (X == 2) t = fma((R)8.0, v[H + 1] - v[H - 1], v[H - 2] - v[H + 2]) / (R)12.0;
+        else             t = fma((R)45.0, v[H + 1] - v[H - 1], fma((R)-9.0, v[H + 2] - v[H - 2], v[H + 3] - v[H - 3])) / (R)60.0;
         return div_const(t, h, ih);
     }
     if (hi && X >= n - 4) {
@@ -475,9 +468,8 @@ __device__ __forceinline__ R d0bw(const R *v, const D0<R> &c, int X, int n, bool
         const int q = X - n;
         if (q == -1)      t = (v[H] - v[H - 1]);
         else if (q == -2) t = (v[H + 1] - v[H - 1]) * (R)0.5;
-        else if (q == -3) t = (v[H - 2] - (R)8.0 * v[H - 1] + (R)8.0 * v[H + 1] - v[H + 2]) / (R)12.0;
-        else              t = (v[H + 3] - v[H - 3] - (R)9.0 * (v[H + 2] - v[H - 2])
-                              + (R)45.0 * (v[H + 1] - v[H - 1])) / (R)60.0;
+        else if (q == -3) t = fma((R)8.0, v[H + 1] - v[H - 1], v[H - 2] - v[H + 2]) / (R)12.0;
+        else              t = fma((R)45.0, v[H + 1] - v[H - 1], fma((R)-9.0, v[H + 2] - v[H - 2], v[H + 3] - v[H - 3])) / (R)60.0;
         return div_const(t, h, ih);
     }
     return d0w<R, H>(v, c);
@@ -615,7 +607,7 @@ k_vdiv(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tmx
 #pragma unroll
                 for (int dd = 0; dd < 3; dd++)
 #pragma unroll
-                    for (int m = 0; m < 4; m++) acc[m + 1] += ajac * dv[dd][m];
+                    for (int m = 0; m < 4; m++) acc[m + 1] = fma(ajac, dv[dd][m], acc[m + 1]);
                 double a64[5];
 #pragma unroll
                 for (int m = 0; m < 5; m++) a64[m] = (double)acc[m];
@@ -712,9 +704,9 @@ k_vev(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tmq,
             }
             if (valid && !failed) {
                 const long long o = lap_index(p, i + OCFD_LAP, j + OCFD_LAP, k + OCFD_LAP);
-                R Akx = (R)metric<UNI>(p, M_AKX, o), Aix = (R)metric<UNI>(p, M_AIX, o), Asx = (R)metric<UNI>(p, M_ASX, o);
-                R Aky = (R)metric<UNI>(p, M_AKY, o), Aiy = (R)metric<UNI>(p, M_AIY, o), Asy = (R)metric<UNI>(p, M_ASY, o);
-                R Akz = (R)metric<UNI>(p, M_AKZ, o), Aiz = (R)metric<UNI>(p, M_AIZ, o), Asz = (R)metric<UNI>(p, M_ASZ, o);
+                R m[3][3];                            // [direction][component]
+#pragma unroll
+                for (int q = 0; q < 9; q++) m[q / 3][q % 3] = (R)metric<UNI>(p, M_AKX + q, o);
                 R Tc = at(k, 3, 0, 0);
                 R Amu = (R)p.amu_C0 * sqrt_r(Tc * Tc * Tc) / ((R)p.Tsb + Tc);      // get_Amu_kernal
                 const D0<R> cx(p, 0), cy(p, 1), cz(p, 2);
@@ -738,45 +730,8 @@ k_vev(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tmq,
                         ds[f] = d0bw<R, H>(vz, cz, k, p.nz, p.bnd_lo[2], p.bnd_hi[2]);
                     }
                 }
-                const R uk = dk[0], ui = di[0], us = ds[0], vk = dk[1], vi = di[1], vs = ds[1];
-                const R wk = dk[2], wi = di[2], ws = ds[2], Tk = dk[3], Ti = di[3], Ts = ds[3];
-                R ux = uk*Akx + ui*Aix + us*Asx;
-                R vx = vk*Akx + vi*Aix + vs*Asx;
-                R wx = wk*Akx + wi*Aix + ws*Asx;
-                R uy = uk*Aky + ui*Aiy + us*Asy;
-                R vy = vk*Aky + vi*Aiy + vs*Asy;
-                R wy = wk*Aky + wi*Aiy + ws*Asy;
-                R uz = uk*Akz + ui*Aiz + us*Asz;
-                R vz = vk*Akz + vi*Aiz + vs*Asz;
-                R wz = wk*Akz + wi*Aiz + ws*Asz;
-                R div = ux + vy + wz;
-                R s11 = ((R)2.0*ux - (R)(2.0/3.0)*div) * Amu;
-                R s22 = ((R)2.0*vy - (R)(2.0/3.0)*div) * Amu;
-                R s33 = ((R)2.0*wz - (R)(2.0/3.0)*div) * Amu;
-                R s12 = (uy + vx) * Amu;
-                R s13 = (uz + wx) * Amu;
-                R s23 = (vz + wy) * Amu;
-                R uu = at(k, 0, 0, 0), vv = at(k, 1, 0, 0), ww = at(k, 2, 0, 0);
-                R Amuk = Amu * (R)p.vis_c;
-                R Tx = Tk*Akx + Ti*Aix + Ts*Asx;
-                R Ty = Tk*Aky + Ti*Aiy + Ts*Asy;
-                R Tz = Tk*Akz + Ti*Aiz + Ts*Asz;
-                R E1 = uu*s11 + vv*s12 + ww*s13 + Amuk*Tx;
-                R E2 = uu*s12 + vv*s22 + ww*s23 + Amuk*Ty;
-                R E3 = uu*s13 + vv*s23 + ww*s33 + Amuk*Tz;
-                R Aj1 = (R)metric<UNI>(p, M_AJAC, o);
-                R *const evb = ev_r<R>(p);
-#pragma unroll
-                for (int dd = 0; dd < 3; dd++) {
-                    R akx = (R)metric<UNI>(p, M_AKX + 3 * dd, o) * Aj1;
-                    R aky = (R)metric<UNI>(p, M_AKX + 3 * dd + 1, o) * Aj1;
-                    R akz = (R)metric<UNI>(p, M_AKX + 3 * dd + 2, o) * Aj1;
-                    R *ev = evb + (long long)(4 * dd) * p.lapN;
-                    ev[o]              = (akx*s11 + aky*s12 + akz*s13);
-                    ev[p.lapN + o]     = (akx*s12 + aky*s22 + akz*s23);
-                    ev[2 * p.lapN + o] = (akx*s13 + aky*s23 + akz*s33);
-                    ev[3 * p.lapN + o] = (akx*E1  + aky*E2  + akz*E3);
-                }
+                vis_fluxes<UNI, R>(p, o, m, Amu, dk[0], di[0], ds[0], dk[1], di[1], ds[1], dk[2], di[2], ds[2],
+                                   dk[3], di[3], ds[3], at(k, 0, 0, 0), at(k, 1, 0, 0), at(k, 2, 0, 0));
             }
             if (__syncthreads_or(failed)) { failed = true; break; }
             if (k + H + 2 <= k1 - 1 + H) {          // into the slot of plane k-H, read for the last time
