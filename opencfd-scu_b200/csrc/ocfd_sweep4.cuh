@@ -36,10 +36,17 @@ __device__ __forceinline__ R rv(const R *ring, int col, int sv, int Q) {
     return ring[(sv * RING + ring_slot<RING>(Q)) * LC + col];
 }
 
-// lines, and points of the ring, a warp: a pass's window of LY + 7 points
-// fits the ring exactly enough for five blocks of the y and z walks an SM
-template <int DIR> struct Shape4 { static constexpr int LC = 8, RING = 12; };
-template <> struct Shape4<0> { static constexpr int LC = 1, RING = 64; };
+// lines, and points of the ring, a warp: a pass's window of LY + 7 points fits
+// the ring, and five blocks of the y and z walks an SM.  In x the faces of
+// four rows share a warp (a row of 512 takes 65 passes of 8 a lane group, where
+// 32 of one row would take 17 of them four times over with a nearly empty last);
+// WENO7's shorter faces gain nothing from it and keep one row.
+template <int DIR, int KIND> struct Shape4 {
+    static constexpr int LC = DIR == 0 ? (KIND == K_W7 ? 1 : 4) : 8, RING = DIR == 0 ? (KIND == K_W7 ? 64 : 16) : 12;
+};
+
+// distance of a face's values in the face buffer
+template <int LC> __device__ __forceinline__ constexpr int fb_stride() { return (32 / LC + 1) * LC; }
 
 // One sign of a characteristic face F+1/2: the sign's 7-point stencil of
 // the five split fields, projected on each characteristic field, the
@@ -51,7 +58,7 @@ template <> struct Shape4<0> { static constexpr int LC = 1, RING = 64; };
 // stays small; otherwise the general form (WENO7 or WENO5, closures)
 template <int S, int RING, int LC, bool HOT, typename R>
 __device__ __forceinline__ void char_sign(const R *ring, int col, int F, int n, bool w7, bool near,
-                                          bool lo, bool hi, const R (&rec)[FP_N], R (&out)[10]) {
+                                          bool lo, bool hi, const R (&rec)[FP_N], R *fb) {
     constexpr int K0 = S, K1 = S + 6;
     R fv[5][8];
 #pragma unroll
@@ -93,7 +100,7 @@ __device__ __forceinline__ void char_sign(const R *ring, int col, int F, int n, 
         for (int c = 0; c < 5; c++) one(c);
     }
 #pragma unroll
-    for (int m = 0; m < 5; m++) out[S * 5 + m] = o5[m];
+    for (int m = 0; m < 5; m++) fb[(S * 5 + m) * fb_stride<LC>()] = o5[m];
 }
 
 // A face on the flux components with a boundary closure in reach: W7 picks
@@ -101,7 +108,7 @@ __device__ __forceinline__ void char_sign(const R *ring, int col, int F, int n, 
 // of each sign.
 template <int RING, int LC, bool W7, typename R>
 __device__ __forceinline__ void comp_face_closure(const R *ring, int col, int F, int n, bool lo, bool hi,
-                                                  int KA0, int KB0, int KA1, int KB1, R *out) {
+                                                  int KA0, int KB0, int KA1, int KB1, R *fb) {
     for (int sv = 0; sv < 10; sv++) {
         const int sign = sv >= 5;
         R vals[8];
@@ -112,19 +119,19 @@ __device__ __forceinline__ void comp_face_closure(const R *ring, int col, int F,
             if (W7) r = sign ? weno7_m(vals) : weno7_p(vals);
             else    r = sign ? up7_m_q(vals) : up7_p_q(vals);
         }
-        out[sv] = r;
+        fb[sv * fb_stride<LC>()] = r;
     }
 }
 
 template <int RING, int LC, typename R>
-__device__ __forceinline__ void face_w7(const R *ring, int col, int F, R (&out)[10]) {
+__device__ __forceinline__ void face_w7(const R *ring, int col, int F, R *fb) {
 #pragma unroll
     for (int sv = 0; sv < 10; sv++) {
         R vals[8];
 #pragma unroll
         for (int k = 0; k < 8; k++)
             vals[k] = (sv < 5 ? k < 7 : k > 0) ? rv<RING, LC>(ring, col, sv, F - 3 + k) : (R)0.0;
-        out[sv] = sv < 5 ? weno7_p(vals) : weno7_m(vals);
+        fb[sv * fb_stride<LC>()] = sv < 5 ? weno7_p(vals) : weno7_m(vals);
     }
 }
 
@@ -138,26 +145,29 @@ __device__ __forceinline__ void face_w7(const R *ring, int col, int F, R (&out)[
 template <int KIND, int RING, int LC, bool UNI, bool SPLIT, typename R>
 __device__ __forceinline__ void face4(const Params &p, int dir, const R *ring, int col, int F, int n,
                                       int hflag, long long o0, long long sd, bool lo, bool hi,
-                                      R (&out)[10]) {
+                                      R *fb) {
     const bool near = (lo && F <= 3) || (hi && F >= n - 5);
     if (near && (KIND == K_W7 || hflag == 1)) {
-        R tmp[10];
-        if (KIND == K_W7) comp_face_closure<RING, LC, true>(ring, col, F, n, lo, hi, 3, 3, 3, 3, tmp);
-        else              comp_face_closure<RING, LC, false>(ring, col, F, n, lo, hi, 3, 4, 4, 3, tmp);
-#pragma unroll
-        for (int sv = 0; sv < 10; sv++) out[sv] = tmp[sv];
+        if (KIND == K_W7) comp_face_closure<RING, LC, true>(ring, col, F, n, lo, hi, 3, 3, 3, 3, fb);
+        else              comp_face_closure<RING, LC, false>(ring, col, F, n, lo, hi, 3, 4, 4, 3, fb);
         return;
     }
-    if (KIND == K_W7) { face_w7<RING, LC>(ring, col, F, out); return; }
-    if (hflag == 1) { face_up7<RING, LC>(ring, col, F, out); return; }
+    if (KIND == K_W7) { face_w7<RING, LC>(ring, col, F, fb); return; }
+    if (hflag == 1) {
+        R out[10];
+        face_up7<RING, LC>(ring, col, F, out);
+#pragma unroll
+        for (int sv = 0; sv < 10; sv++) fb[sv * fb_stride<LC>()] = out[sv];
+        return;
+    }
     R rec[FP_N];
     face_record<UNI>(p, dir, o0, o0 + sd, rec);
     if (SPLIT && hflag == 2 && !near) {
-        char_sign<0, RING, LC, true>(ring, col, F, n, true, false, lo, hi, rec, out);
-        char_sign<1, RING, LC, true>(ring, col, F, n, true, false, lo, hi, rec, out);
+        char_sign<0, RING, LC, true>(ring, col, F, n, true, false, lo, hi, rec, fb);
+        char_sign<1, RING, LC, true>(ring, col, F, n, true, false, lo, hi, rec, fb);
     } else {
-        char_sign<0, RING, LC, false>(ring, col, F, n, hflag == 2, near, lo, hi, rec, out);
-        char_sign<1, RING, LC, false>(ring, col, F, n, hflag == 2, near, lo, hi, rec, out);
+        char_sign<0, RING, LC, false>(ring, col, F, n, hflag == 2, near, lo, hi, rec, fb);
+        char_sign<1, RING, LC, false>(ring, col, F, n, hflag == 2, near, lo, hi, rec, fb);
     }
 }
 
@@ -228,14 +238,15 @@ __device__ __forceinline__ void du_rule_cell(const Params &p, const R *ring, int
 // left from the buffer.
 template <int DIR, bool UNI, bool EPS0, int KIND, int MINB, bool SPLIT, typename R>
 __global__ void __launch_bounds__(32 * SW, MINB) k_sweep4(const __grid_constant__ Params p, int seg_len) {
-    constexpr int LC = Shape4<DIR>::LC, LY = 32 / LC, RING = Shape4<DIR>::RING, FR = LY + 1;
+    constexpr int LC = Shape4<DIR, KIND>::LC, LY = 32 / LC, RING = Shape4<DIR, KIND>::RING, FR = LY + 1;
     static_assert(LY + 7 <= RING, "a pass's window fits the ring");
     extern __shared__ __align__(16) unsigned char smem4[];   // per warp: ring, then face buffer
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int col = lane % LC, ly = lane / LC;
     const long long grp = (long long)blockIdx.x * SW + wid;     // line group of this warp
     const int ngx = (p.nx + LC - 1) / LC;
-    const long long ngroups = DIR == 0 ? (long long)p.ny * p.nz : (long long)ngx * (DIR == 1 ? p.nz : p.ny);
+    const long long nrows = (long long)p.ny * p.nz;
+    const long long ngroups = DIR == 0 ? (nrows + LC - 1) / LC : (long long)ngx * (DIR == 1 ? p.nz : p.ny);
     if (grp >= ngroups) return;                                 // the whole warp
     R *ring = reinterpret_cast<R *>(smem4) + (size_t)wid * 10 * (RING + FR) * LC;
     R *fbuf = ring + 10 * RING * LC;
@@ -247,11 +258,13 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep4(const __grid_constant_
     const int8_t *fl;
     bool colok = true;
     if (DIR == 0) {
-        const int j = (int)(grp % p.ny), k = (int)(grp / p.ny);
+        colok = grp * LC + col < nrows;
+        const long long row = colok ? grp * LC + col : nrows - 1;  // keep addresses in range
+        const int j = (int)(row % p.ny), k = (int)(row / p.ny);
         base = (long long)(k + OCFD_LAP) * p.zs + (long long)(j + OCFD_LAP) * p.ys + OCFD_LAP;
         sd = 1;
-        cb = in_index(p, 0, j, k); cst = 1;
-        fl = p.flag[0] + (long long)(p.nx + 1) * ((long long)j + (long long)p.ny * k); fst = 1;
+        cb = (long long)p.nx * row; cst = 1;
+        fl = p.flag[0] + (long long)(p.nx + 1) * row; fst = 1;
     } else {
         const int x = (int)(grp % ngx) * LC + col, c3 = (int)(grp / ngx);
         colok = x < p.nx;
@@ -295,17 +308,17 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep4(const __grid_constant_
         }
         const int hflag = (KIND == K_HYBC && valid) ? flag_at(p, DIR, fl, (long long)(F + 1) * fst) : 2;
         __syncwarp();
-        R cur[10];
-        if (valid) {
-            face4<KIND, RING, LC, UNI, SPLIT>(p, DIR, ring, col, F, n, hflag, base + (long long)F * sd, sd, lo, hi, cur);
-#pragma unroll
-            for (int sv = 0; sv < 10; sv++) fbuf[(sv * FR + ly + 1) * LC + col] = cur[sv];
-        }
+        if (valid)
+            face4<KIND, RING, LC, UNI, SPLIT>(p, DIR, ring, col, F, n, hflag, base + (long long)F * sd, sd, lo, hi,
+                                              fbuf + (ly + 1) * LC + col);
         __syncwarp();
         if (valid && F >= y0) {
-            R prv[10];
+            R cur[10], prv[10];
 #pragma unroll
-            for (int sv = 0; sv < 10; sv++) prv[sv] = fbuf[(sv * FR + ly) * LC + col];
+            for (int sv = 0; sv < 10; sv++) {
+                prv[sv] = fbuf[(sv * FR + ly) * LC + col];
+                cur[sv] = fbuf[(sv * FR + ly + 1) * LC + col];
+            }
             const long long ci = OCFD_IDX(p, cb + (long long)F * cst, N);
             const R aj = (R)metric<UNI>(p, M_AJAC, base + (long long)F * sd);
             if (p.has_bnd && rule_cell(p, DIR, F, n)) {
@@ -324,7 +337,7 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep4(const __grid_constant_
         __syncwarp();
         if (valid && ly == LY - 1) {
 #pragma unroll
-            for (int sv = 0; sv < 10; sv++) fbuf[sv * FR * LC + col] = cur[sv];
+            for (int sv = 0; sv < 10; sv++) fbuf[sv * FR * LC + col] = fbuf[(sv * FR + LY) * LC + col];
         }
     }
 }
@@ -474,20 +487,14 @@ __global__ void __launch_bounds__(32 * FIX4W) k_sweep4_fix(const __grid_constant
 
 template <int DIR, bool UNI, bool EPS0, int KIND, int MINB, bool SPLIT, typename R>
 cudaError_t launch_dir4(const Params &p, cudaStream_t st) {
-    constexpr int LC = Shape4<DIR>::LC, LY = 32 / LC;
+    constexpr int LC = Shape4<DIR, KIND>::LC, LY = 32 / LC;
     const int n = DIR == 0 ? p.nx : (DIR == 1 ? p.ny : p.nz);
     const long long ngx = (p.nx + LC - 1) / LC;
-    const long long groups = DIR == 0 ? (long long)p.ny * p.nz : ngx * (DIR == 1 ? p.nz : p.ny);
+    const long long groups = DIR == 0 ? ((long long)p.ny * p.nz + LC - 1) / LC : ngx * (DIR == 1 ? p.nz : p.ny);
     const int seg_len = segment_cells(groups, n, LY, 148LL * MINB * SW, 3);
     dim3 grid((unsigned)((groups + SW - 1) / SW), (unsigned)((n + seg_len - 1) / seg_len));
-    constexpr int smem = SW * 10 * (Shape4<DIR>::RING + LY + 1) * LC * (int)sizeof(R);
-    static bool attr_set = false;             // above the 48 KB default
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(k_sweep4<DIR, UNI, EPS0, KIND, MINB, SPLIT, R>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-        attr_set = true;
-    }
+    constexpr int smem = SW * 10 * (Shape4<DIR, KIND>::RING + LY + 1) * LC * (int)sizeof(R);
+    static_assert(smem <= 48 * 1024, "no attribute needed");
     k_sweep4<DIR, UNI, EPS0, KIND, MINB, SPLIT, R><<<grid, 32 * SW, smem, st>>>(p, seg_len);
     return cudaGetLastError();
 }
@@ -503,7 +510,7 @@ cudaError_t dir4s(const Params &p, int dir, cudaStream_t st) {
 }
 template <bool UNI, bool EPS0, int KIND, typename R>
 cudaError_t dir4k(const Params &p, int dir, cudaStream_t st) {
-    if (KIND == K_HYBC && !p.has_bnd) return dir4s<UNI, EPS0, KIND, true, R>(p, dir, st);
+    if constexpr (KIND == K_HYBC) if (!p.has_bnd) return dir4s<UNI, EPS0, KIND, true, R>(p, dir, st);
     return dir4s<UNI, EPS0, KIND, false, R>(p, dir, st);
 }
 
