@@ -272,44 +272,33 @@ __device__ __forceinline__ double weno7_m(const double *s8) {
     return weno7_core(v);
 }
 
-// WENO5 positive side, src/OCFD_Schemes.cu:1118-1151; q = s+1 (f(F-2..F+2))
-__device__ __forceinline__ double weno5_p(const double *s8) {
-    const double *s = s8 + 1;
-    double S0 = 0.0, S1 = 0.0, S2 = 0.0, tmp;
-    const double ep = 1e-6;
-    tmp =     s[2] - 2.0*s[3] + s[4]; S0 += 13*tmp*tmp;
-    tmp = 3.0*s[2] - 4.0*s[3] + s[4]; S0 +=  3*tmp*tmp;
-    double q03 = (2.0*s[2] + 5.0*s[3] - s[4]);
-    tmp = s[1] - 2.0*s[2] + s[3]; S1 += 13*tmp*tmp;
-    tmp =                  s[1] - s[3]; S1 +=  3*tmp*tmp;
-    double q13 = (-s[1] + 5.0*s[2] + 2.0*s[3]);
-    tmp = s[0] - 2.0*s[1] +     s[2]; S2 += 13*tmp*tmp;
-    tmp = s[0] - 4.0*s[1] + 3.0*s[2]; S2 +=  3*tmp*tmp;
-    double q23 = (2.0*s[0] - 7.0*s[1] + 11.0*s[2]);
-    double a0 = 3.0*((12.0*ep + S1)*(12.0*ep + S1))*((12.0*ep + S2)*(12.0*ep + S2));
-    double a1 = 6.0*((12.0*ep + S0)*(12.0*ep + S0))*((12.0*ep + S2)*(12.0*ep + S2));
-    double a2 =     ((12.0*ep + S0)*(12.0*ep + S0))*((12.0*ep + S1)*(12.0*ep + S1));
-    return (a0*q03 + a1*q13 + a2*q23)/(6.0*(a0 + a1 + a2));
+// WENO5 of a stencil in upwind order (v[1..5]; P: src/OCFD_Schemes.cu:1118-1151,
+// M: :1176-1208) over the candidates of mask (bit 0: v[3..5], 1: v[2..4], 2:
+// v[1..3]); the boundary closures take fewer than all (src/OCFD_bound_Scheme.cu:554-745).
+// Differences as in Diff7, candidates as their distance from v[3].  FP32
+// forms the weights as one quotient each, where the common denominator could overflow.
+template <typename R>
+__device__ __forceinline__ R weno5_core(const R *v, int mask = 7) {
+    const R d1 = v[2] - v[1], d2 = v[3] - v[2], d3 = v[4] - v[3], d4 = v[5] - v[4];
+    const R e1 = d2 - d1, e2 = d3 - d2, e3 = d4 - d3;
+    auto beta = [](R g, R t) { return fma((R)13.0 * g, g, fma((R)3.0 * t, t, (R)(12.0 * 1e-6))); };
+    R b0 = beta(e3, fma((R)-2.0, d3, e3)), b1 = beta(e2, d2 + d3), b2 = beta(e1, fma((R)2.0, d2, e1));
+    // (a candidate left out takes no part in the common denominator)
+    b0 = mask & 1 ? b0 * b0 : (R)1.0; b1 = mask & 2 ? b1 * b1 : (R)1.0; b2 = mask & 4 ? b2 * b2 : (R)1.0;
+    const R k0 = mask & 1 ? (R)3.0 : (R)0.0, k1 = mask & 2 ? (R)6.0 : (R)0.0, k2 = mask & 4 ? (R)1.0 : (R)0.0;
+    R a0, a1, a2;
+    if constexpr (sizeof(R) == 8) {
+        a0 = k0 * b1 * b2; a1 = k1 * b0 * b2; a2 = k2 * b0 * b1;
+    } else {
+        a0 = k0 / b0; a1 = k1 / b1; a2 = k2 / b2;
+    }
+    const R q0 = fma((R)3.0, d3, -e3), q1 = fma((R)2.0, d3, d2), q2 = fma((R)2.0, e1, (R)3.0 * d2);
+    return v[3] + fma(a0, q0, fma(a1, q1, a2 * q2)) / ((R)6.0 * (a0 + a1 + a2));
 }
-
-// WENO5 negative side, src/OCFD_Schemes.cu:1176-1208; q = s+2 (f(F-1..F+3))
+__device__ __forceinline__ double weno5_p(const double *s) { return weno5_core(s); }
 __device__ __forceinline__ double weno5_m(const double *s8) {
-    const double *s = s8 + 2;
-    double S0 = 0.0, S1 = 0.0, S2 = 0.0, tmp;
-    const double ep = 1e-6;
-    tmp =     s[2] - 2.0*s[1] + s[0]; S0 += 13*tmp*tmp;
-    tmp = 3.0*s[2] - 4.0*s[1] + s[0]; S0 +=  3*tmp*tmp;
-    double q03 = (2.0*s[2] + 5.0*s[1] - s[0]);
-    tmp = s[3] - 2.0*s[2] + s[1]; S1 += 13*tmp*tmp;
-    tmp =                  s[3] - s[1]; S1 +=  3*tmp*tmp;
-    double q13 = (-s[3] + 5.0*s[2] + 2.0*s[1]);
-    tmp = s[4] - 2.0*s[3] +     s[2]; S2 += 13*tmp*tmp;
-    tmp = s[4] - 4.0*s[3] + 3.0*s[2]; S2 +=  3*tmp*tmp;
-    double q23 = (2.0*s[4] - 7.0*s[3] + 11.0*s[2]);
-    double a0 = 3.0*((12.0*ep + S1)*(12.0*ep + S1))*((12.0*ep + S2)*(12.0*ep + S2));
-    double a1 = 6.0*((12.0*ep + S0)*(12.0*ep + S0))*((12.0*ep + S2)*(12.0*ep + S2));
-    double a2 =     ((12.0*ep + S0)*(12.0*ep + S0))*((12.0*ep + S1)*(12.0*ep + S1));
-    return (a0*q03 + a1*q13 + a2*q23)/(6.0*(a0 + a1 + a2));
+    const double v[6] = { s8[7], s8[6], s8[5], s8[4], s8[3], s8[2] };
+    return weno5_core(v);
 }
 
 // UP7, src/OCFD_Schemes.cu:865-907

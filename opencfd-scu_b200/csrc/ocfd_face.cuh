@@ -169,116 +169,43 @@ __device__ __forceinline__ double recon_one(const Params &p, int scheme, int hfl
     }
 }
 
-// one-sided WENO5 candidates used by the closures, src/OCFD_bound_Scheme.cu:554-745;
-// s[0..4] = f(i-2..i+2)
-__device__ __forceinline__ double w5_p_left(const double *s) {
-    double S0 = 0.0, tmp; const double ep = 1e-6;
-    tmp = s[2] - 2.0*s[3] + s[4]; S0 += 13*tmp*tmp;
-    tmp = 3.0*s[2] - 4.0*s[3] + s[4]; S0 += 3*tmp*tmp;
-    double a0 = 1.0/((12.0*ep + S0)*(12.0*ep + S0));
-    double q03 = (2.0*s[2] + 5.0*s[3] - s[4]);
-    return a0*q03/(6.0*a0);
-}
-__device__ __forceinline__ double w5_m_left(const double *s) {
-    double S2 = 0.0, tmp; const double ep = 1e-6;
-    tmp = s[4] - 2.0*s[3] + s[2]; S2 += 13*tmp*tmp;
-    tmp = s[4] - 4.0*s[3] + 3.0*s[2]; S2 += 3*tmp*tmp;
-    double a2 = 1.0/((12.0*ep + S2)*(12.0*ep + S2));
-    double q23 = (2.0*s[4] - 7.0*s[3] + 11.0*s[2]);
-    return a2*q23/(6.0*a2);
-}
-__device__ __forceinline__ double w5_p_right_plus(const double *s) {
-    double S1 = 0.0, S2 = 0.0, tmp; const double ep = 1e-6;
-    tmp = s[1] - 2.0*s[2] + s[3]; S1 += 13*tmp*tmp;
-    tmp = s[1] - s[3]; S1 += 3*tmp*tmp;
-    double a1 = 6.0/((12.0*ep + S1)*(12.0*ep + S1));
-    double q13 = (-s[1] + 5.0*s[2] + 2.0*s[3]);
-    tmp = s[0] - 2.0*s[1] + s[2]; S2 += 13*tmp*tmp;
-    tmp = s[0] - 4.0*s[1] + 3.0*s[2]; S2 += 3*tmp*tmp;
-    double a2 = 1.0/((12.0*ep + S2)*(12.0*ep + S2));
-    double q23 = (2.0*s[0] - 7.0*s[1] + 11.0*s[2]);
-    return (a1*q13 + a2*q23)/(6.0*(a1 + a2));
-}
-__device__ __forceinline__ double w5_p_left_plus(const double *s) {
-    double S0 = 0.0, S1 = 0.0, tmp; const double ep = 1e-6;
-    tmp = s[2] - 2.0*s[3] + s[4]; S0 += 13*tmp*tmp;
-    tmp = 3.0*s[2] - 4.0*s[3] + s[4]; S0 += 3*tmp*tmp;
-    double a0 = 3.0/((12.0*ep + S0)*(12.0*ep + S0));
-    double q03 = (2.0*s[2] + 5.0*s[3] - s[4]);
-    tmp = s[1] - 2.0*s[2] + s[3]; S1 += 13*tmp*tmp;
-    tmp = s[1] - s[3]; S1 += 3*tmp*tmp;
-    double a1 = 6.0/((12.0*ep + S1)*(12.0*ep + S1));
-    double q13 = (-s[1] + 5.0*s[2] + 2.0*s[3]);
-    return (a0*q03 + a1*q13)/(6.0*(a0 + a1));
-}
-__device__ __forceinline__ double w5_m_right_plus(const double *s) {
-    double S0 = 0.0, S1 = 0.0, tmp; const double ep = 1e-6;
-    tmp = s[2] - 2.0*s[1] + s[0]; S0 += 13*tmp*tmp;
-    tmp = 3.0*s[2] - 4.0*s[1] + s[0]; S0 += 3*tmp*tmp;
-    double a0 = 3.0/((12.0*ep + S0)*(12.0*ep + S0));
-    double q03 = (2.0*s[2] + 5.0*s[1] - s[0]);
-    tmp = s[3] - 2.0*s[2] + s[1]; S1 += 13*tmp*tmp;
-    tmp = s[3] - s[1]; S1 += 3*tmp*tmp;
-    double a1 = 6.0/((12.0*ep + S1)*(12.0*ep + S1));
-    double q13 = (-s[3] + 5.0*s[2] + 2.0*s[1]);
-    return (a0*q03 + a1*q13)/(6.0*(a0 + a1));
-}
-__device__ __forceinline__ double w5_m_left_plus(const double *s) {
-    double S1 = 0.0, S2 = 0.0, tmp; const double ep = 1e-6;
-    tmp = s[3] - 2.0*s[2] + s[1]; S1 += 13*tmp*tmp;
-    tmp = s[3] - s[1]; S1 += 3*tmp*tmp;
-    double a1 = 6.0/((12.0*ep + S1)*(12.0*ep + S1));
-    double q13 = (-s[3] + 5.0*s[2] + 2.0*s[1]);
-    tmp = s[4] - 2.0*s[3] + s[2]; S2 += 13*tmp*tmp;
-    tmp = s[4] - 4.0*s[3] + 3.0*s[2]; S2 += 3*tmp*tmp;
-    double a2 = 1.0/((12.0*ep + S2)*(12.0*ep + S2));
-    double q23 = (2.0*s[4] - 7.0*s[3] + 11.0*s[2]);
-    return (a1*q13 + a2*q23)/(6.0*(a1 + a2));
-}
-
-// Closure of face F+1/2 of a line of n cells, v[t] = f(F-3+t); returns true
-// when it replaces the interior scheme (OCFD_bound_scheme_kernel_p / _m with
-// boundp1/boundp2/boundm1/boundm2, :748-944).  KA, KB: stencil extents
-// (-ia1, ib1) of the reference kernel of this sign.
-__device__ __forceinline__ bool closure(int sign, bool lo, bool hi, int KA, int KB, int F, int n,
-                                        const double *v, double &out) {
-    int c = F + 1;
+// Closure of face F+1/2 of a line of n cells (OCFD_bound_scheme_kernel_p / _m
+// with boundp1/boundp2/boundm1/boundm2, src/OCFD_bound_Scheme.cu:554-944): 0
+// where the interior scheme stands, bits 0 to 2 the candidates of a WENO5 over
+// part of its stencil, CL_* the formulas beside the boundary.  KA, KB: stencil
+// extents (-ia1, ib1) of the reference kernel of this sign.  A class is
+// found once for a face; its fields then share one reconstruction body.
+enum { CL_DOWN = 8, CL_UP = 16, CL_MID = 32 };
+__device__ __forceinline__ int closure_class(int sign, bool lo, bool hi, int KA, int KB, int F, int n) {
+    const int c = F + 1, t = c - (n + 1);
     if (sign == 0) {
-        if (lo && c <= KA) {
-            if (c == 0) out = v[4];
-            else if (c == 1) out = w5_p_left(v + 1);
-            else if (c == 2) out = w5_p_left_plus(v + 1);
-            else out = weno5_p(v);
-            return true;
-        }
-        if (hi) {
-            int t = c - (n + 1);
-            if (t >= -KB) {
-                if (t == -1) out = v[3] + 0.5 * minmod2(v[3] - v[2], v[3] - v[2]);
-                else if (t == -2) out = w5_p_right_plus(v + 1);
-                else out = weno5_p(v);
-                return true;
-            }
-        }
-        return false;
+        if (lo && c <= KA) return c == 0 ? CL_DOWN : c == 1 ? 1 : c == 2 ? 3 : 7;
+        if (hi && t >= -KB) return t == -1 ? CL_UP : t == -2 ? 6 : 7;
+    } else {
+        if (lo && c < KA) return c == 0 ? 4 : c == 1 ? 6 : 7;
+        if (hi && t >= -KB - 1) return t == -1 ? CL_DOWN : t == -2 ? CL_MID : t == -3 ? 3 : 7;
     }
-    if (lo && c < KA) {
-        if (c == 0) out = w5_m_left(v + 2);
-        else if (c == 1) out = w5_m_left_plus(v + 2);
-        else out = weno5_m(v);
-        return true;
-    }
-    if (hi) {
-        int t = c - (n + 1);
-        if (t >= -KB - 1) {
-            if (t == -1) out = v[3];
-            else if (t == -2) out = v[4] - 0.5 * minmod2(v[4] - v[3], v[4] - v[3]);
-            else if (t == -3) out = w5_m_right_plus(v + 2);
-            else out = weno5_m(v);
-            return true;
-        }
-    }
-    return false;
+    return 0;
+}
+// its value from the stencil in upwind order (v[3] the upwind cell).  The
+// limited differences beside the boundary are of one difference with itself.
+template <typename R>
+__device__ __forceinline__ R closure_value(int cls, const R *v) {
+    R r = weno5_core(v, cls & 7);
+    if (cls >= CL_DOWN)
+        r = cls == CL_DOWN ? v[4] : cls == CL_UP ? v[3] + (R)0.5 * (v[3] - v[2]) : v[3] + (R)0.5 * (v[4] - v[3]);
+    return r;
+}
+// v[t] = f(F-3+t); true when the closure replaces the interior scheme
+template <typename R>
+__device__ __forceinline__ bool closure(int sign, bool lo, bool hi, int KA, int KB, int F, int n, const R *v, R &out) {
+    const int cls = closure_class(sign, lo, hi, KA, KB, F, n);
+    if (!cls) return false;
+    R u[6];
+#pragma unroll
+    for (int t = 0; t < 6; t++) u[t] = sign ? v[7 - t] : v[t];
+    out = closure_value(cls, u);
+    return true;
 }
 
 // stencil extents of the reference kernels per scheme and sign (P: -ia1, ib1)

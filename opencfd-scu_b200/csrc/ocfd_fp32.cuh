@@ -134,128 +134,15 @@ __device__ __forceinline__ float weno7_m(const float *s8) {
     return weno7_core(v);
 }
 
-// WENO5 (positive side uses s8[1..5], negative side s8[2..6])
-__device__ __forceinline__ float weno5_p(const float *s8) {
-    const float *s = s8 + 1;
-    const float ep = 1e-6f;
-    float t = s[2] - 2.0f*s[3] + s[4], u = 3.0f*s[2] - 4.0f*s[3] + s[4];
-    const float S0 = 13.0f*t*t + 3.0f*u*u;
-    t = s[1] - 2.0f*s[2] + s[3]; u = s[1] - s[3];
-    const float S1 = 13.0f*t*t + 3.0f*u*u;
-    t = s[0] - 2.0f*s[1] + s[2]; u = s[0] - 4.0f*s[1] + 3.0f*s[2];
-    const float S2 = 13.0f*t*t + 3.0f*u*u;
-    const float a0 = fdiv(3.0f, (12.0f*ep + S0) * (12.0f*ep + S0));
-    const float a1 = fdiv(6.0f, (12.0f*ep + S1) * (12.0f*ep + S1));
-    const float a2 = fdiv(1.0f, (12.0f*ep + S2) * (12.0f*ep + S2));
-    const float q03 = 2.0f*s[2] + 5.0f*s[3] - s[4];
-    const float q13 = -s[1] + 5.0f*s[2] + 2.0f*s[3];
-    const float q23 = 2.0f*s[0] - 7.0f*s[1] + 11.0f*s[2];
-    return fdiv(a0*q03 + a1*q13 + a2*q23, 6.0f*(a0 + a1 + a2));
-}
+__device__ __forceinline__ float weno5_p(const float *s) { return weno5_core(s); }
 __device__ __forceinline__ float weno5_m(const float *s8) {
-    const float *s = s8 + 2;
-    const float ep = 1e-6f;
-    float t = s[2] - 2.0f*s[1] + s[0], u = 3.0f*s[2] - 4.0f*s[1] + s[0];
-    const float S0 = 13.0f*t*t + 3.0f*u*u;
-    t = s[3] - 2.0f*s[2] + s[1]; u = s[3] - s[1];
-    const float S1 = 13.0f*t*t + 3.0f*u*u;
-    t = s[4] - 2.0f*s[3] + s[2]; u = s[4] - 4.0f*s[3] + 3.0f*s[2];
-    const float S2 = 13.0f*t*t + 3.0f*u*u;
-    const float a0 = fdiv(3.0f, (12.0f*ep + S0) * (12.0f*ep + S0));
-    const float a1 = fdiv(6.0f, (12.0f*ep + S1) * (12.0f*ep + S1));
-    const float a2 = fdiv(1.0f, (12.0f*ep + S2) * (12.0f*ep + S2));
-    const float q03 = 2.0f*s[2] + 5.0f*s[1] - s[0];
-    const float q13 = -s[3] + 5.0f*s[2] + 2.0f*s[1];
-    const float q23 = 2.0f*s[4] - 7.0f*s[3] + 11.0f*s[2];
-    return fdiv(a0*q03 + a1*q13 + a2*q23, 6.0f*(a0 + a1 + a2));
+    const float v[6] = { s8[7], s8[6], s8[5], s8[4], s8[3], s8[2] };
+    return weno5_core(v);
 }
 
 __device__ __forceinline__ float sgn1(float x2) { return x2 >= 0 ? 1.0f : -1.0f; }
 __device__ __forceinline__ float minmod2(float x1, float x2) {
     return 0.5f*(sgn1(x1) + sgn1(x2))*fminf(fabsf(x1), fabsf(x2));
-}
-
-// one-sided WENO5 candidates of the boundary closures; s[0..4] = f(i-2..i+2)
-__device__ __forceinline__ float w5_beta(float t, float u) { return 13.0f*t*t + 3.0f*u*u; }
-// single-candidate closures: the candidate's weight cancels
-__device__ __forceinline__ float w5_p_left(const float *s) {
-    return (2.0f*s[2] + 5.0f*s[3] - s[4]) / 6.0f;
-}
-__device__ __forceinline__ float w5_m_left(const float *s) {
-    return (2.0f*s[4] - 7.0f*s[3] + 11.0f*s[2]) / 6.0f;
-}
-__device__ __forceinline__ float w5_pair(float a, float qa, float b, float qb) {
-    return (a*qa + b*qb) / (6.0f*(a + b));
-}
-__device__ __forceinline__ float w5_p_right_plus(const float *s) {
-    const float ep12 = 12.0e-6f;
-    const float S1 = w5_beta(s[1] - 2.0f*s[2] + s[3], s[1] - s[3]);
-    const float S2 = w5_beta(s[0] - 2.0f*s[1] + s[2], s[0] - 4.0f*s[1] + 3.0f*s[2]);
-    return w5_pair(6.0f / ((ep12 + S1)*(ep12 + S1)), -s[1] + 5.0f*s[2] + 2.0f*s[3],
-                   1.0f / ((ep12 + S2)*(ep12 + S2)), 2.0f*s[0] - 7.0f*s[1] + 11.0f*s[2]);
-}
-__device__ __forceinline__ float w5_p_left_plus(const float *s) {
-    const float ep12 = 12.0e-6f;
-    const float S0 = w5_beta(s[2] - 2.0f*s[3] + s[4], 3.0f*s[2] - 4.0f*s[3] + s[4]);
-    const float S1 = w5_beta(s[1] - 2.0f*s[2] + s[3], s[1] - s[3]);
-    return w5_pair(3.0f / ((ep12 + S0)*(ep12 + S0)), 2.0f*s[2] + 5.0f*s[3] - s[4],
-                   6.0f / ((ep12 + S1)*(ep12 + S1)), -s[1] + 5.0f*s[2] + 2.0f*s[3]);
-}
-__device__ __forceinline__ float w5_m_right_plus(const float *s) {
-    const float ep12 = 12.0e-6f;
-    const float S0 = w5_beta(s[2] - 2.0f*s[1] + s[0], 3.0f*s[2] - 4.0f*s[1] + s[0]);
-    const float S1 = w5_beta(s[3] - 2.0f*s[2] + s[1], s[3] - s[1]);
-    return w5_pair(3.0f / ((ep12 + S0)*(ep12 + S0)), 2.0f*s[2] + 5.0f*s[1] - s[0],
-                   6.0f / ((ep12 + S1)*(ep12 + S1)), -s[3] + 5.0f*s[2] + 2.0f*s[1]);
-}
-__device__ __forceinline__ float w5_m_left_plus(const float *s) {
-    const float ep12 = 12.0e-6f;
-    const float S1 = w5_beta(s[3] - 2.0f*s[2] + s[1], s[3] - s[1]);
-    const float S2 = w5_beta(s[4] - 2.0f*s[3] + s[2], s[4] - 4.0f*s[3] + 3.0f*s[2]);
-    return w5_pair(6.0f / ((ep12 + S1)*(ep12 + S1)), -s[3] + 5.0f*s[2] + 2.0f*s[1],
-                   1.0f / ((ep12 + S2)*(ep12 + S2)), 2.0f*s[4] - 7.0f*s[3] + 11.0f*s[2]);
-}
-
-// boundary closure of face F+1/2 (the FP64 closure() with these candidates)
-__device__ __forceinline__ bool closure(int sign, bool lo, bool hi, int KA, int KB, int F, int n,
-                                        const float *v, float &out) {
-    int c = F + 1;
-    if (sign == 0) {
-        if (lo && c <= KA) {
-            if (c == 0) out = v[4];
-            else if (c == 1) out = w5_p_left(v + 1);
-            else if (c == 2) out = w5_p_left_plus(v + 1);
-            else out = weno5_p(v);
-            return true;
-        }
-        if (hi) {
-            int t = c - (n + 1);
-            if (t >= -KB) {
-                if (t == -1) out = v[3] + 0.5f * minmod2(v[3] - v[2], v[3] - v[2]);
-                else if (t == -2) out = w5_p_right_plus(v + 1);
-                else out = weno5_p(v);
-                return true;
-            }
-        }
-        return false;
-    }
-    if (lo && c < KA) {
-        if (c == 0) out = w5_m_left(v + 2);
-        else if (c == 1) out = w5_m_left_plus(v + 2);
-        else out = weno5_m(v);
-        return true;
-    }
-    if (hi) {
-        int t = c - (n + 1);
-        if (t >= -KB - 1) {
-            if (t == -1) out = v[3];
-            else if (t == -2) out = v[4] - 0.5f * minmod2(v[4] - v[3], v[4] - v[3]);
-            else if (t == -3) out = w5_m_right_plus(v + 2);
-            else out = weno5_m(v);
-            return true;
-        }
-    }
-    return false;
 }
 
 // characteristic eigen-rows from a face record in FP32 (layout of FP_N)

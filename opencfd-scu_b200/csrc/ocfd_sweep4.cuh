@@ -53,12 +53,11 @@ template <int LC> __device__ __forceinline__ constexpr int fb_stride() { return 
 // reconstruction (or the boundary closure) and the back-projection, with
 // the operations and order of face_generic.  Point F-3+k is stencil entry k;
 // sign 0 uses entries 0..6, sign 1 entries 1..7.
-// HOT: a WENO7 face with no closure in reach -- the common case on grids
-// without closed faces, kept compact so the loop's instruction footprint
-// stays small; otherwise the general form (WENO7 or WENO5, closures)
+// cls: 0 WENO7, else the class of a closure or of WENO5 (closure_class).
+// HOT: WENO7 alone -- the common case on grids without closed faces, kept
+// compact so the loop's instruction footprint stays small
 template <int S, int RING, int LC, bool HOT, typename R>
-__device__ __forceinline__ void char_sign(const R *ring, int col, int F, int n, bool w7, bool near,
-                                          bool lo, bool hi, const R (&rec)[FP_N], R *fb) {
+__device__ __forceinline__ void char_sign(const R *ring, int col, int F, int cls, const R (&rec)[FP_N], R *fb) {
     constexpr int K0 = S, K1 = S + 6;
     R fv[5][8];
 #pragma unroll
@@ -68,16 +67,14 @@ __device__ __forceinline__ void char_sign(const R *ring, int col, int F, int n, 
             fv[m][k] = (k >= K0 && k <= K1) ? rv<RING, LC>(ring, col, S * 5 + m, F - 3 + k) : (R)0.0;
     R o5[5];
     auto one = [&](int c) {
-        R Lr[5], vals[8], Rc[5];
+        R Lr[5], v[7], Rc[5];                // v: upwind order
         L_row(rec, 1, c, Lr);
 #pragma unroll
-        for (int k = 0; k < 8; k++)
-            vals[k] = (k >= K0 && k <= K1) ? dot5(Lr, fv[0][k], fv[1][k], fv[2][k], fv[3][k], fv[4][k]) : (R)0.0;
-        R res;
-        if (HOT)
-            res = S ? weno7_m(vals) : weno7_p(vals);
-        else if (!(near && closure(S, lo, hi, S ? 4 : 3, S ? 3 : 4, F, n, vals, res)))
-            res = w7 ? (S ? weno7_m(vals) : weno7_p(vals)) : (S ? weno5_m(vals) : weno5_p(vals));
+        for (int t = 0; t < 7; t++) {
+            const int k = S ? 7 - t : t;
+            v[t] = dot5(Lr, fv[0][k], fv[1][k], fv[2][k], fv[3][k], fv[4][k]);
+        }
+        const R res = HOT || cls == 0 ? weno7_core(v) : closure_value(cls, v);
         R_col(rec, 1, c, Rc);
         if (c == 0) {
 #pragma unroll
@@ -163,11 +160,13 @@ __device__ __forceinline__ void face4(const Params &p, int dir, const R *ring, i
     R rec[FP_N];
     face_record<UNI>(p, dir, o0, o0 + sd, rec);
     if (SPLIT && hflag == 2 && !near) {
-        char_sign<0, RING, LC, true>(ring, col, F, n, true, false, lo, hi, rec, fb);
-        char_sign<1, RING, LC, true>(ring, col, F, n, true, false, lo, hi, rec, fb);
+        char_sign<0, RING, LC, true>(ring, col, F, 0, rec, fb);
+        char_sign<1, RING, LC, true>(ring, col, F, 0, rec, fb);
     } else {
-        char_sign<0, RING, LC, false>(ring, col, F, n, hflag == 2, near, lo, hi, rec, fb);
-        char_sign<1, RING, LC, false>(ring, col, F, n, hflag == 2, near, lo, hi, rec, fb);
+        const int other = hflag == 2 ? 0 : 7;         // WENO7, or WENO5 over its whole stencil
+        const int c0 = near ? closure_class(0, lo, hi, 3, 4, F, n) : 0, c1 = near ? closure_class(1, lo, hi, 4, 3, F, n) : 0;
+        char_sign<0, RING, LC, false>(ring, col, F, c0 ? c0 : other, rec, fb);
+        char_sign<1, RING, LC, false>(ring, col, F, c1 ? c1 : other, rec, fb);
     }
 }
 
