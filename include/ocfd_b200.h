@@ -102,22 +102,17 @@ int ocfd_b200_set_metrics(ocfd_b200_ctx *ctx, const double *metrics13);
 int ocfd_b200_set_metric_mode(ocfd_b200_ctx *ctx, int mode);
 int ocfd_b200_uniform_metrics(const ocfd_b200_ctx *ctx);
 /* Inviscid sweep kernel variant: 4 (default) no block barriers: each warp
- * walks its own lines (one x row, or 8 y or z lines) through a ring of
- * split values in shared memory.  For UP7 the loop makes no calls and the
- * cells at bounded line ends are finished by a second kernel with the same
- * arithmetic; for WENO7 and the characteristic hybrid scheme every face,
- * closure and line-end rule is formed in the walk (variant 6), except that a
- * hybrid direction whose sensor pass marked almost every face UP7 takes the
- * UP7 walk with its few other cells deferred (the choice is read back once
- * per step, after the sensor); in the precision form the y and z UP7 walks
- * run as per-lane marches over pencil tiles staged in shared memory by the
- * tensor copy engine, each lane keeping its face window in registers.
- * 5: the walk with every face through one in-loop dispatch (the path of the
- * schemes other than UP7, WENO7 and the hybrid scheme in variant 4 too);
+ * walks its own lines (4 x rows, or 8 y or z lines) through a ring of split
+ * values in shared memory and forms every face, closure and line-end rule
+ * in the walk; UP7, and a hybrid direction whose sensor pass marked almost
+ * every face UP7 (the choice is read back once per step, after the sensor),
+ * take the UP7 walk: rows of four cells a lane in x, per-lane marches in y and
+ * z, the few cells beside other faces finished by a second kernel.
+ * 5: the generic walk, every face through one in-loop dispatch (variant 4
+ * where projection is asked of a scheme that has none);
  * 6: the in-line walk alone (characteristic hybrid scheme and WENO7 only);
- * 7: as 4 with the y and z UP7 walks through the shared-memory ring; 8: as 4
- * (it once chose the marches in FP64, which 4 now takes too).  All
- * agree to the parity bound (WENO weights amplify the different multiply-add
+ * 7: as 4 with the y and z UP7 walks through the shared-memory ring; 8: as 4.
+ * All agree to the parity bound (WENO weights amplify the different multiply-add
  * contractions); 4, 7 and 8 agree bit for bit.  Other values: OCFD_ERR_ARG. */
 int ocfd_b200_set_sweep_impl(ocfd_b200_ctx *ctx, int impl);
 /* Arithmetic form of the stencils.  0 (default): FP64 throughout, the

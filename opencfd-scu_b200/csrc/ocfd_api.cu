@@ -60,6 +60,7 @@ int reduce_scratch_doubles();
 cudaError_t launch_sweeps3(const Params &p, cudaStream_t st);
 cudaError_t launch_sweeps4(const Params &p, cudaStream_t st);
 bool sweeps4_supported(const Params &p);
+bool sweeps4_covers(const Params &p);
 cudaError_t launch_sweep4_dir(const Params &p, int dir, cudaStream_t st);
 cudaError_t launch_sweep3_dir(const Params &p, int dir, cudaStream_t st);
 bool sweeps3_defers(const Params &p);
@@ -637,9 +638,9 @@ static bool walk4_wanted(const ocfd_b200_ctx *ctx, int d, unsigned nonup7) {
 
 static int sweeps_auto(ocfd_b200_ctx *ctx) {
     const Params &p = ctx->p;
-    const bool hyb = p.scheme_invis == 310;
+    const bool hyb = p.scheme_invis == 310 && p.charteric;
     int w[3];
-    for (int d = 0; d < 3; d++) w[d] = (hyb && p.sweep_impl != 6) ? ctx->walk4[d] : 1;
+    for (int d = 0; d < 3; d++) w[d] = (hyb && p.sweep_impl != 6) ? ctx->walk4[d] : ocfd::sweeps4_covers(p);
     if ((!w[0] || !w[1] || !w[2]) && ocfd::sweeps3_defers(p))
         CK(cudaMemsetAsync(p.defer_count, 0, 3 * sizeof(unsigned), ctx->stream), "deferred counters");
     for (int d = 0; d < 3; d++) {
@@ -726,7 +727,7 @@ static int rhs(ocfd_b200_ctx *ctx, int krk, int fused_rk, bool skip_sensor = fal
         TimerScope ts(ctx, T_SWEEP);
         if (p.sweep_impl == 6 && !ocfd::sweeps4_supported(p))
             return fail(ctx, OCFD_ERR_UNSUPPORTED, "sweep variant 6 covers the characteristic hybrid scheme and WENO7");
-        if (p.mixed || (p.sweep_impl == 4 && ocfd::sweeps4_supported(p))) {
+        if (p.mixed || (p.sweep_impl == 4 && (ocfd::sweeps4_covers(p) || ocfd::march_supported(p, 1)))) {
             int rc = sweeps_auto(ctx);
             if (rc) return rc;
         } else {            // the other variants launch the three directions together

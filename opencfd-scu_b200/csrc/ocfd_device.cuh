@@ -325,14 +325,14 @@ __device__ __forceinline__ double minmod4(double x1, double x2, double x3, doubl
     return m*t;
 }
 
-// NND2, src/OCFD_Schemes.cu:800-837: P uses f(F-1..F+1), M uses f(F..F+2)
-__device__ __forceinline__ double nnd2_p(const double *s8) {
-    const double *s = s8 + 2;
-    return s[1] + 0.5*minmod2(s[2] - s[1], s[1] - s[0]);
+// NND2 of a stencil in upwind order, src/OCFD_Schemes.cu:800-837
+__device__ __forceinline__ double nnd2_up(const double *v) {
+    return v[3] + 0.5*minmod2(v[4] - v[3], v[3] - v[2]);
 }
+__device__ __forceinline__ double nnd2_p(const double *s8) { return nnd2_up(s8); }
 __device__ __forceinline__ double nnd2_m(const double *s8) {
-    const double *s = s8 + 3;
-    return s[1] + 0.5*minmod2(s[0] - s[1], s[1] - s[2]);
+    const double v[5] = { 0.0, 0.0, s8[5], s8[4], s8[3] };
+    return nnd2_up(v);
 }
 
 __device__ __forceinline__ void omp6_mn(int flag, double &m, double &n) {
@@ -341,84 +341,48 @@ __device__ __forceinline__ void omp6_mn(int flag, double &m, double &n) {
     else { m = 0.015; n = 0.0; }
 }
 
-// OMP6 positive side, src/OCFD_Schemes.cu:936-1008
-__device__ __forceinline__ double omp6_p(int flag, const double *s) {
-    double m, n; omp6_mn(flag, m, n);
-    double mid_nf = 0.5*(m + n); m = 0.5*(m - n);
-    mid_nf =             ( 60.0*mid_nf  * s[7] +
-      ( 1.0 -   60.0*m -  360.0*mid_nf) * s[6] +
-      (-8.0 +  360.0*m +  900.0*mid_nf) * s[5] +
-      (37.0 -  900.0*m - 1200.0*mid_nf) * s[4] +
-      (37.0 + 1200.0*m +  900.0*mid_nf) * s[3] +
-      (-8.0 -  900.0*m -  360.0*mid_nf) * s[2] +
-      (1.0  +  360.0*m +   60.0*mid_nf) * s[1] -
-                                 60.0*m * s[0])/60.0;
-    m = s[3] + minmod2((s[4] - s[3]), (s[3] - s[2]));
-    if ((mid_nf - s[3])*(mid_nf - m) >= 1.e-10) {
-        double tmp, tmp1;
-        m = s[2] + s[4] - 2.0*s[3];
-        n = s[3] + s[5] - 2.0*s[4];
-        tmp = 4.0*m - n;
-        tmp1 = 4.0*n - m;
-        tmp = 0.5*(s[3] + s[4]) - 0.5*minmod4(tmp, tmp1, n, m);
-        n = s[1] + s[3] - 2.0*s[2];
-        tmp1 = s[3] + 0.5*(s[3] - s[2]) + 4.0*minmod4(4*n - m, 4*m - n, m, n)/3.0;
-        double lo, hi;
-        {
-            lo = fmin(fmin(s[3], s[4]), tmp);
-            double q = s[3] + 4.0*(s[3] - s[2]);
-            q = fmin(fmin(s[3], q), tmp1);
-            lo = fmax(lo, q);
-        }
-        {
-            double t2 = fmax(s[4], fmax(s[3], tmp));
-            double q = s[3] + 4.0*(s[3] - s[2]);
-            q = fmax(fmax(s[3], q), tmp1);
-            hi = fmin(t2, q);
-        }
-        mid_nf = mid_nf + minmod2(hi - mid_nf, lo - mid_nf);
+// OMP6, src/OCFD_Schemes.cu:972-1095: coefficients of the linear flux (times 60) ...
+struct Omp6 {
+    double c[8];
+    __device__ __forceinline__ explicit Omp6(int flag) {
+        double m, n;
+        omp6_mn(flag, m, n);
+        const double mid = 0.5*(m + n);
+        m = 0.5*(m - n);
+        c[0] = -60.0*m;
+        c[1] = 1.0 + 360.0*m + 60.0*mid;
+        c[2] = -8.0 - 900.0*m - 360.0*mid;
+        c[3] = 37.0 + 1200.0*m + 900.0*mid;
+        c[4] = 37.0 - 900.0*m - 1200.0*mid;
+        c[5] = -8.0 + 360.0*m + 900.0*mid;
+        c[6] = 1.0 - 60.0*m - 360.0*mid;
+        c[7] = 60.0*mid;
     }
-    return mid_nf;
+};
+// ... and the limited value of a stencil in upwind order.  The negative side
+// (S = 1) takes its large-curvature bound from the downwind difference and
+// the point behind the cell in its lower bound.
+template <int S>
+__device__ __forceinline__ double omp6_up(const Omp6 &k, const double *v) {
+    double f = k.c[7]*v[7] + k.c[6]*v[6] + k.c[5]*v[5] + k.c[4]*v[4] + k.c[3]*v[3] + k.c[2]*v[2] + k.c[1]*v[1] + k.c[0]*v[0];
+    f = div_const(f, 60.0, 1.0 / 60.0);
+    const double mp = v[3] + minmod2(v[4] - v[3], v[3] - v[2]);
+    if ((f - v[3])*(f - mp) >= 1.e-10) {
+        const double c0 = v[2] + v[4] - 2.0*v[3], c1 = v[3] + v[5] - 2.0*v[4], cm = v[1] + v[3] - 2.0*v[2];
+        const double md = 0.5*(v[3] + v[4]) - 0.5*minmod4(4.0*c0 - c1, 4.0*c1 - c0, c1, c0);
+        const double lc = v[3] + 0.5*(S ? v[3] - v[4] : v[3] - v[2])
+                        + div_const(4.0*minmod4(4.0*cm - c0, 4.0*c0 - cm, c0, cm), 3.0, 1.0 / 3.0);
+        const double ul = v[3] + 4.0*(v[3] - v[2]);
+        const double lo = fmax(fmin(fmin(S ? v[2] : v[3], v[4]), md), fmin(fmin(v[3], ul), lc));
+        const double hi = fmin(fmax(v[4], fmax(v[3], md)), fmax(fmax(v[3], ul), lc));
+        f = f + minmod2(hi - f, lo - f);
+    }
+    return f;
 }
-
-// OMP6 negative side, src/OCFD_Schemes.cu:1037-1095 (s = f(F-3..F+4))
-__device__ __forceinline__ double omp6_m(int flag, const double *s) {
-    double m, n; omp6_mn(flag, m, n);
-    double mid_nf = 0.5*(m + n); m = 0.5*(m - n);
-    mid_nf =            (  60.0*mid_nf  * s[0] +
-       (1.0 -   60.0*m -  360.0*mid_nf) * s[1] +
-      (-8.0 +  360.0*m +  900.0*mid_nf) * s[2] +
-      (37.0 -  900.0*m - 1200.0*mid_nf) * s[3] +
-      (37.0 + 1200.0*m +  900.0*mid_nf) * s[4]  +
-      (-8.0 -  900.0*m -  360.0*mid_nf) * s[5]  +
-       (1.0 +  360.0*m +   60.0*mid_nf) * s[6]  -
-                                 60.0*m * s[7])/60.0;
-    m = s[4] + minmod2((s[3] - s[4]), (s[4] - s[5]));
-    if ((mid_nf - s[4])*(mid_nf - m) >= 1.e-10) {
-        double tmp, tmp1;
-        m = s[5] + s[3] - 2.0*s[4];
-        n = s[4] + s[2] - 2.0*s[3];
-        tmp = 4.0*m - n;
-        tmp1 = 4.0*n - m;
-        tmp = 0.5*(s[4] + s[3]) - 0.5*minmod4(tmp, tmp1, n, m);
-        n = s[6] + s[4] - 2.0*s[5];
-        tmp1 = s[4] + 0.5*(s[4] - s[3]) + 4.0*minmod4(4*n - m, 4*m - n, m, n)/3.0;
-        double lo, hi;
-        {
-            lo = fmin(fmin(s[5], s[3]), tmp);
-            double q = s[4] + 4.0*(s[4] - s[5]);
-            q = fmin(fmin(s[4], q), tmp1);
-            lo = fmax(lo, q);
-        }
-        {
-            double t2 = fmax(s[3], fmax(s[4], tmp));
-            double q = s[4] + 4.0*(s[4] - s[5]);
-            q = fmax(fmax(s[4], q), tmp1);
-            hi = fmin(t2, q);
-        }
-        mid_nf = mid_nf + minmod2(hi - mid_nf, lo - mid_nf);
-    }
-    return mid_nf;
+__device__ __forceinline__ double omp6_p(int flag, const double *s) { return omp6_up<0>(Omp6(flag), s); }
+__device__ __forceinline__ double omp6_m(int flag, const double *s8) {
+    const double v[8] = { s8[7], s8[6], s8[5], s8[4], s8[3], s8[2], s8[1], s8[0] };
+    return omp6_up<1>(Omp6(flag), v);
 }
 
 // WENO7-SYMBO weights and reconstruction, shared by both signs once the

@@ -1,22 +1,25 @@
 // ocfd_sweep4.cuh -- inviscid flux sweeps with every face formed in the walk
-// (sm_100a, FP64).
+// (sm_100a).
 //
 // Same results as the walk of ocfd_sweep3.cu, and so as the reference's
-// OCFD_d{x,y,z}1/2 chain, for the two schemes whose faces are mostly not UP7:
+// OCFD_d{x,y,z}1/2 chain, for the schemes whose faces are mostly not UP7:
 //   K_HYBC  the hybrid scheme with its auto sensor and characteristic
 //           projection (src/OCFD_Schemes_hybrid_auto.cu:862-1023 with
 //           src/OCFD_flux_charteric.cu:330-752): a flag-1 face takes UP7 on
 //           each flux component, a flag-2 face WENO7 and any other face WENO5
 //           on the characteristic fields;
-//   K_W7    WENO7 on each flux component (src/OCFD_Schemes.cu:640-741).
+//   K_HYBN  the same by flux components, each by the face's flag or the one
+//           the parameters give for components 1 to 4;
+//   K_SYMC  WENO7-SYMBO, limited or not, on the characteristic fields;
+//   K_W7, K_W5, K_SYM, K_OMP6, K_NND2  the scheme on each flux component.
 // Nothing goes out of line and no cell is left for a second kernel: one
 // sign's stencil of a characteristic face (7 points x 5 fields) and the
 // face's eigen-record are held in registers, and the boundary closures and
 // the first/last-cell rules of bounded lines are applied where they fall.
 // The fluxes of one pass go to a per-warp face buffer in shared memory, from
 // which each lane takes the flux of the face on its left.
-// (Templates; ocfd_sweep4.cu instantiates them in FP64, ocfd_sweep4_f32.cu in
-// FP32 for the precision form.)
+// (Templates; ocfd_sweep4.cu and the ocfd_sweep4_*.cu beside it instantiate
+// them in FP64, ocfd_sweep4_f32.cu in FP32 for the precision form.)
 #pragma once
 #include "ocfd_walk.cuh"
 
@@ -28,7 +31,9 @@ namespace walk4 {
 
 using namespace walk;
 
-enum { K_HYBC = 0, K_W7 = 1 };
+enum { K_HYBC = 0, K_W7, K_HYBN, K_SYMC, K_W5, K_SYM, K_OMP6, K_NND2 };
+constexpr bool char_kind(int k) { return k == K_HYBC || k == K_SYMC; }
+constexpr bool flag_kind(int k) { return k == K_HYBC || k == K_HYBN; }
 
 // ring value sv of point Q of line col
 template <int RING, int LC, typename R>
@@ -45,6 +50,12 @@ template <int DIR, int KIND> struct Shape4 {
     static constexpr int LC = DIR == 0 ? (KIND == K_W7 ? 1 : 4) : 8, RING = DIR == 0 ? (KIND == K_W7 ? 64 : 16) : 12;
 };
 
+// SYMBO of a stencil in upwind order (the negative side never takes its linear weights)
+template <int S>
+__device__ __forceinline__ double symbo_up(const Params &p, const double *v) {
+    return S ? symbo_core(false, v) : symbo_p(p.scheme_invis == 305, p.tv_lim, p.tv_max, v);
+}
+
 // distance of a face's values in the face buffer
 template <int LC> __device__ __forceinline__ constexpr int fb_stride() { return (32 / LC + 1) * LC; }
 
@@ -56,9 +67,11 @@ template <int LC> __device__ __forceinline__ constexpr int fb_stride() { return 
 // cls: 0 WENO7, else the class of a closure or of WENO5 (closure_class).
 // HOT: WENO7 alone -- the common case on grids without closed faces, kept
 // compact so the loop's instruction footprint stays small
-template <int S, int RING, int LC, bool HOT, typename R>
-__device__ __forceinline__ void char_sign(const R *ring, int col, int F, int cls, const R (&rec)[FP_N], R *fb) {
-    constexpr int K0 = S, K1 = S + 6;
+template <int KIND, int S, int RING, int LC, bool HOT, typename R>
+__device__ __forceinline__ void char_sign(const Params &p, const R *ring, int col, int F, int cls,
+                                          const R (&rec)[FP_N], R *fb) {
+    constexpr int NP = KIND == K_SYMC ? 8 : 7;       // points of the scheme's stencil, from the upwind end
+    constexpr int K0 = NP == 8 ? 0 : S, K1 = NP == 8 ? 7 : S + 6;
     R fv[5][8];
 #pragma unroll
     for (int m = 0; m < 5; m++)
@@ -67,14 +80,16 @@ __device__ __forceinline__ void char_sign(const R *ring, int col, int F, int cls
             fv[m][k] = (k >= K0 && k <= K1) ? rv<RING, LC>(ring, col, S * 5 + m, F - 3 + k) : (R)0.0;
     R o5[5];
     auto one = [&](int c) {
-        R Lr[5], v[7], Rc[5];                // v: upwind order
+        R Lr[5], v[NP], Rc[5];               // v: upwind order
         L_row(rec, 1, c, Lr);
 #pragma unroll
-        for (int t = 0; t < 7; t++) {
+        for (int t = 0; t < NP; t++) {
             const int k = S ? 7 - t : t;
             v[t] = dot5(Lr, fv[0][k], fv[1][k], fv[2][k], fv[3][k], fv[4][k]);
         }
-        const R res = HOT || cls == 0 ? weno7_core(v) : closure_value(cls, v);
+        R res;
+        if constexpr (KIND == K_SYMC) res = cls == 0 ? symbo_up<S>(p, v) : closure_value(cls, v);
+        else                          res = HOT || cls == 0 ? weno7_core(v) : closure_value(cls, v);
         R_col(rec, 1, c, Rc);
         if (c == 0) {
 #pragma unroll
@@ -132,6 +147,33 @@ __device__ __forceinline__ void face_w7(const R *ring, int col, int F, R *fb) {
     }
 }
 
+// A face on the flux components, sign by sign and field by field in one body
+// of the scheme: unrolled, ten copies of it wait on instruction fetch.
+template <int KIND, int S, int RING, int LC>
+__device__ __forceinline__ void comp_sign(const Params &p, const double *ring, int col, int F, int cls, int hflag,
+                                          double *fb) {
+    int at[8];
+#pragma unroll
+    for (int t = 0; t < 8; t++) at[t] = ring_slot<RING>(S ? F + 4 - t : F - 3 + t) * LC + col;
+    const Omp6 omp(p.scheme_invis - 307);
+#pragma unroll 1
+    for (int m = 0; m < 5; m++) {
+        double v[8], r;                       // upwind order
+#pragma unroll
+        for (int t = 0; t < 8; t++) v[t] = ring[(S * 5 + m) * RING * LC + at[t]];
+        if (cls) r = closure_value(cls, v);
+        else if constexpr (KIND == K_W5) r = weno5_core(v);
+        else if constexpr (KIND == K_SYM) r = symbo_up<S>(p, v);
+        else if constexpr (KIND == K_NND2) r = nnd2_up(v);
+        else if constexpr (KIND == K_OMP6) r = omp6_up<S>(omp, v);
+        else {
+            const int q = m > 0 && p.nochar_comp_flag ? p.nochar_comp_flag : hflag;
+            r = q == 1 ? up7_p_q(v) : q == 2 ? weno7_core(v) : weno5_core(v);
+        }
+        fb[(S * 5 + m) * fb_stride<LC>()] = r;
+    }
+}
+
 // Flux of face F+1/2 (both signs, all fields) of one lane's line.  Every
 // path is in line: a call here, even on the rare closure faces alone,
 // makes the walk keep its loop state in local memory around it.
@@ -144,13 +186,20 @@ __device__ __forceinline__ void face4(const Params &p, int dir, const R *ring, i
                                       int hflag, long long o0, long long sd, bool lo, bool hi,
                                       R *fb) {
     const bool near = (lo && F <= 3) || (hi && F >= n - 5);
-    if (near && (KIND == K_W7 || hflag == 1)) {
+    if constexpr (!char_kind(KIND) && KIND != K_W7) {
+        constexpr int KA0 = KIND == K_W5 || KIND == K_NND2 ? 2 : 3, KB0 = KA0 == 2 ? 2 : 4;     // extents()
+        constexpr int KA1 = KB0, KB1 = KA0;
+        comp_sign<KIND, 0, RING, LC>(p, ring, col, F, near ? closure_class(0, lo, hi, KA0, KB0, F, n) : 0, hflag, fb);
+        comp_sign<KIND, 1, RING, LC>(p, ring, col, F, near ? closure_class(1, lo, hi, KA1, KB1, F, n) : 0, hflag, fb);
+        return;
+    } else {
+    if (near && (KIND == K_W7 || (KIND == K_HYBC && hflag == 1))) {
         if (KIND == K_W7) comp_face_closure<RING, LC, true>(ring, col, F, n, lo, hi, 3, 3, 3, 3, fb);
         else              comp_face_closure<RING, LC, false>(ring, col, F, n, lo, hi, 3, 4, 4, 3, fb);
         return;
     }
     if (KIND == K_W7) { face_w7<RING, LC>(ring, col, F, fb); return; }
-    if (hflag == 1) {
+    if (KIND == K_HYBC && hflag == 1) {
         R out[10];
         face_up7<RING, LC>(ring, col, F, out);
 #pragma unroll
@@ -160,13 +209,14 @@ __device__ __forceinline__ void face4(const Params &p, int dir, const R *ring, i
     R rec[FP_N];
     face_record<UNI>(p, dir, o0, o0 + sd, rec);
     if (SPLIT && hflag == 2 && !near) {
-        char_sign<0, RING, LC, true>(ring, col, F, 0, rec, fb);
-        char_sign<1, RING, LC, true>(ring, col, F, 0, rec, fb);
+        char_sign<KIND, 0, RING, LC, true>(p, ring, col, F, 0, rec, fb);
+        char_sign<KIND, 1, RING, LC, true>(p, ring, col, F, 0, rec, fb);
     } else {
-        const int other = hflag == 2 ? 0 : 7;         // WENO7, or WENO5 over its whole stencil
+        const int other = KIND == K_SYMC || hflag == 2 ? 0 : 7;     // the scheme, or WENO5 over its whole stencil
         const int c0 = near ? closure_class(0, lo, hi, 3, 4, F, n) : 0, c1 = near ? closure_class(1, lo, hi, 4, 3, F, n) : 0;
-        char_sign<0, RING, LC, false>(ring, col, F, c0 ? c0 : other, rec, fb);
-        char_sign<1, RING, LC, false>(ring, col, F, c1 ? c1 : other, rec, fb);
+        char_sign<KIND, 0, RING, LC, false>(p, ring, col, F, c0 ? c0 : other, rec, fb);
+        char_sign<KIND, 1, RING, LC, false>(p, ring, col, F, c1 ? c1 : other, rec, fb);
+    }
     }
 }
 
@@ -179,7 +229,7 @@ template <int DIR, int KIND, int RING, int LC, typename R, typename D>
 __device__ __forceinline__ void du_rule_cell(const Params &p, const R *ring, int col, int X, int n,
                                              D *__restrict__ du, long long ci, R aj, R h,
                                              R ih, const R (&cur)[10], const R (&prv)[10]) {
-    constexpr bool char_kernel = KIND == K_HYBC;
+    constexpr bool char_kernel = char_kind(KIND);
     const bool lo = p.bnd_lo[DIR], hi = p.bnd_hi[DIR];
     const bool only_lo = lo && !hi, only_hi = hi && !lo;     // flag 1..6, not 7..9
     const bool first = X == 0, last = X == n - 1;
@@ -305,7 +355,7 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep4(const __grid_constant_
             load5(p, o, q5);
             ring_put<DIR, RING, LC, UNI, EPS0>(p, ring, col, P, o, q5);
         }
-        const int hflag = (KIND == K_HYBC && valid) ? flag_at(p, DIR, fl, (long long)(F + 1) * fst) : 2;
+        const int hflag = (flag_kind(KIND) && valid) ? flag_at(p, DIR, fl, (long long)(F + 1) * fst) : 2;
         __syncwarp();
         if (valid)
             face4<KIND, RING, LC, UNI, SPLIT>(p, DIR, ring, col, F, n, hflag, base + (long long)F * sd, sd, lo, hi,
@@ -498,11 +548,13 @@ cudaError_t launch_dir4(const Params &p, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// FP64: register budget for 3 blocks per SM (characteristic faces), 5 (WENO7);
-// FP32 (the precision form): 4, 5
+// Blocks per SM the registers are fitted to: 5 on the flux components; FP64
+// characteristic faces 3 (ramp 512x128x64, x / y / z: 1149 / 1097 / 1013 us; 2 1280 /
+// 1237 / 1193, 4 1266 / 1264 / 1161), 2 with SYMBO's eight points (176 / 163 / 179 us;
+// 3 178 / 191 / 198), FP32 ones 4 (180 / 179 / 150 us; 5 204 / 181 / 186, 3 220 / 209 / 175)
 template <bool UNI, bool EPS0, int KIND, bool SPLIT, typename R>
 cudaError_t dir4s(const Params &p, int dir, cudaStream_t st) {
-    constexpr int MINB = KIND == K_W7 ? 5 : sizeof(R) == 8 ? 3 : 4;
+    constexpr int MINB = KIND == K_SYMC ? 2 : !char_kind(KIND) ? 5 : sizeof(R) == 8 ? 3 : 4;
     if (dir == 0) return launch_dir4<0, UNI, EPS0, KIND, MINB, SPLIT, R>(p, st);
     if (dir == 1) return launch_dir4<1, UNI, EPS0, KIND, MINB, SPLIT, R>(p, st);
     return launch_dir4<2, UNI, EPS0, KIND, MINB, SPLIT, R>(p, st);
@@ -526,6 +578,13 @@ cudaError_t dir4r(const Params &p, int dir, cudaStream_t st) {
     return dir4<false, false, R>(p, dir, st);
 }
 
+// the other schemes, FP64 only: on a uniform grid with EPSL_SW != 0 they
+// read the metric fields (the same values)
+template <int KIND>
+cudaError_t dir4_more(const Params &p, int dir, cudaStream_t st) {
+    return p.uniform_metrics && p.epsl_sw == 0.0 ? dir4k<true, true, KIND, double>(p, dir, st)
+                                                 : dir4k<false, false, KIND, double>(p, dir, st);
+}
 
 }  // namespace walk4
 }  // namespace ocfd
