@@ -81,7 +81,8 @@ cudaError_t launch_mlp_infer(const float *w, const float *feat, long long n, flo
                              cudaStream_t st);
 cudaError_t launch_mlp_grad(const float *w, const float *feat, const float *label, const int *idx, long long n,
                             float pos_w, float *part, float *lpart, float *grad, double *loss, cudaStream_t st);
-cudaError_t launch_mlp_adam(float *w, const float *grad, float *m1, float *m2, float scale, float lr, int t,
+cudaError_t launch_mlp_step(float *w, const float *feat, const float *label, const int *idx, long long n, float pos_w,
+                            float *part, float *lpart, float *grad, double *loss, float *m1, float *m2, float lr, int t,
                             cudaStream_t st);
 }  // namespace ocfd
 
@@ -1074,22 +1075,23 @@ extern "C" int ocfd_b200_mlp_train(float *params, const float *feat, const float
                                    int batch, float lr, float pos_w, unsigned long long seed, double *epoch_loss) {
     if (!params || !feat || !label || n <= 0 || epochs < 0 || batch <= 0 || n > 0x7fffffffLL) return OCFD_ERR_ARG;
     const int np = ocfd::mlp_nparam(), nn = ocfd::mlp_nnet(), nbmax = ocfd::mlp_grad_blocks(batch);
-    DevBuf w, f, y, part, lpart, g, l, m1, m2, perm;
-    MCK(w.alloc(sizeof(float) * np), "alloc");
-    MCK(f.alloc(sizeof(float) * 14 * (size_t)n), "alloc");
-    MCK(y.alloc(sizeof(float) * (size_t)n), "alloc");
-    MCK(part.alloc(sizeof(float) * (size_t)nbmax * nn), "alloc");
-    MCK(lpart.alloc(sizeof(float) * (size_t)nbmax), "alloc");
-    MCK(g.alloc(sizeof(float) * nn), "alloc");
-    MCK(l.alloc(sizeof(double)), "alloc");
-    MCK(m1.alloc(sizeof(float) * nn), "alloc");
-    MCK(m2.alloc(sizeof(float) * nn), "alloc");
-    MCK(perm.alloc(sizeof(int) * (size_t)n), "alloc");
-    MCK(cudaMemcpy(w.p, params, sizeof(float) * np, cudaMemcpyHostToDevice), "copy");
-    MCK(cudaMemcpy(f.p, feat, sizeof(float) * 14 * (size_t)n, cudaMemcpyHostToDevice), "copy");
-    MCK(cudaMemcpy(y.p, label, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice), "copy");
-    MCK(cudaMemset(m1.p, 0, sizeof(float) * nn), "memset");
-    MCK(cudaMemset(m2.p, 0, sizeof(float) * nn), "memset");
+    // one allocation: the loss, then the arrays, each at a multiple of 256 bytes
+    size_t bytes = 256;
+    auto part_of = [&bytes](size_t b) { const size_t at = bytes; bytes += (b + 255) / 256 * 256; return at; };
+    const size_t f4 = sizeof(float);
+    const size_t ow = part_of(f4 * np), om1 = part_of(f4 * nn), om2 = part_of(f4 * nn), og = part_of(f4 * nn);
+    const size_t of = part_of(f4 * 14 * (size_t)n), oy = part_of(f4 * (size_t)n), op = part_of(f4 * (size_t)nbmax * nn);
+    const size_t ol = part_of(f4 * (size_t)nbmax), oi = part_of(sizeof(int) * (size_t)n);
+    DevBuf buf;
+    MCK(buf.alloc(bytes), "alloc");
+    char *base = buf.as<char>();
+    auto fp = [base](size_t o) { return reinterpret_cast<float *>(base + o); };
+    double *l = reinterpret_cast<double *>(base);
+    int *perm = reinterpret_cast<int *>(base + oi);
+    MCK(cudaMemcpy(fp(ow), params, f4 * np, cudaMemcpyHostToDevice), "copy");
+    MCK(cudaMemcpy(fp(of), feat, f4 * 14 * (size_t)n, cudaMemcpyHostToDevice), "copy");
+    MCK(cudaMemcpy(fp(oy), label, f4 * (size_t)n, cudaMemcpyHostToDevice), "copy");
+    MCK(cudaMemset(fp(om1), 0, og - om1), "memset");
     std::vector<int> order((size_t)n);
     for (long long i = 0; i < n; i++) order[(size_t)i] = (int)i;
     unsigned long long state = seed ? seed : 0x9E3779B97F4A7C15ULL;
@@ -1099,24 +1101,25 @@ extern "C" int ocfd_b200_mlp_train(float *params, const float *feat, const float
         z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
         return z ^ (z >> 31);
     };
-    int t = 0;
-    for (int ep = 0; ep < epochs; ep++) {
+    auto shuffle = [&] {
         for (long long i = n - 1; i > 0; i--) std::swap(order[(size_t)i], order[(size_t)(next() % (unsigned long long)(i + 1))]);
-        MCK(cudaMemcpy(perm.p, order.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice), "copy");
-        MCK(cudaMemset(l.p, 0, sizeof(double)), "memset");
+    };
+    int t = 0;
+    if (epochs > 0) shuffle();
+    for (int ep = 0; ep < epochs; ep++) {
+        MCK(cudaMemcpy(perm, order.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice), "copy");
+        MCK(cudaMemset(l, 0, sizeof(double)), "memset");
         for (long long b0 = 0; b0 < n; b0 += batch) {
             const long long nb = std::min<long long>(batch, n - b0);
-            MCK(ocfd::launch_mlp_grad(w.as<float>(), f.as<float>(), y.as<float>(), perm.as<int>() + b0, nb, pos_w,
-                                      part.as<float>(), lpart.as<float>(), g.as<float>(), l.as<double>(), 0),
-                "mlp_grad");
-            MCK(ocfd::launch_mlp_adam(w.as<float>(), g.as<float>(), m1.as<float>(), m2.as<float>(),
-                                      1.0f / (float)nb, lr, ++t, 0), "mlp_adam");
+            MCK(ocfd::launch_mlp_step(fp(ow), fp(of), fp(oy), perm + b0, nb, pos_w, fp(op), fp(ol), fp(og), l,
+                                      fp(om1), fp(om2), lr, ++t, 0), "mlp_step");
         }
+        if (ep + 1 < epochs) shuffle();          // the next epoch's order, while this one runs
         double ls = 0.0;
-        MCK(cudaMemcpy(&ls, l.p, sizeof(double), cudaMemcpyDeviceToHost), "copy");
+        MCK(cudaMemcpy(&ls, l, sizeof(double), cudaMemcpyDeviceToHost), "copy");
         if (epoch_loss) epoch_loss[ep] = ls / (double)n;
     }
-    MCK(cudaMemcpy(params, w.p, sizeof(float) * np, cudaMemcpyDeviceToHost), "copy");
+    MCK(cudaMemcpy(params, fp(ow), f4 * np, cudaMemcpyDeviceToHost), "copy");
     return OCFD_OK;
 }
 

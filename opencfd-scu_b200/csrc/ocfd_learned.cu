@@ -440,61 +440,70 @@ __global__ void __launch_bounds__(umma::ROWS) k_switch_infer(Params p, const flo
 // ---------------------------------------------------------------------------
 // training (FP32)
 // ---------------------------------------------------------------------------
-constexpr int TB = 64;     // samples (and threads) per block
+constexpr int TB = 64;     // samples per block
+constexpr int TQ = 4;      // threads per sample, MLP_H / TQ neurons each
 
 // Forward and backward pass of TB samples (rows idx[0..], or 0.. when idx is
 // null); writes this block's gradient sums (MLP_NNET values, in the order of
 // the parameter vector from W1) to part[blockIdx.x] and its loss sum to
 // lpart[blockIdx.x].  Loss: BCE with logits, positive samples weighted pos_w.
-__global__ void __launch_bounds__(TB) k_mlp_grad(const float *__restrict__ w, const float *__restrict__ feat,
+// Bound by the length of a thread's chain of sums (a batch of 16384 rows is
+// two blocks an SM): four threads a sample share its neurons, and all the
+// block's outputs: 31 -> 22 us a batch.
+__global__ void __launch_bounds__(TB * TQ) k_mlp_grad(const float *__restrict__ w, const float *__restrict__ feat,
                                                  const float *__restrict__ label, const int *__restrict__ idx,
                                                  long long n, float pos_w, float *__restrict__ part,
                                                  float *__restrict__ lpart) {
     __shared__ float sX[TB][MLP_IN + 1], sH1[TB][MLP_H + 1], sD1[TB][MLP_H + 1], sH2[TB][MLP_H + 1],
         sD2[TB][MLP_H + 1], sD3[TB], sLoss[TB];
-    const int s = threadIdx.x;
+    const int s = threadIdx.x % TB, q = threadIdx.x / TB;     // q is one value a warp
+    const int a0 = q * (MLP_H / TQ), a1 = a0 + MLP_H / TQ;     // this thread's neurons
     const long long row = (long long)blockIdx.x * TB + s;
     const bool live = row < n;
-    // this sample's vectors live in its own rows of the shared arrays; the
-    // ReLU masks are bit masks
+    // a sample's vectors live in its own rows of the shared arrays; the
+    // ReLU masks of the thread's neurons are bit masks
     const long long src = live ? (idx ? (long long)idx[row] : row) : 0;
-    for (int m = 0; m < MLP_IN; m++)
+    for (int m = q; m < MLP_IN; m += TQ)
         sX[s][m] = live ? (feat[src * MLP_IN + m] - w[OFF_MU + m]) / w[OFF_SG + m] : 0.0f;
+    __syncthreads();
     unsigned mask1 = 0u, mask2 = 0u;
 #pragma unroll 4
-    for (int a = 0; a < MLP_H; a++) {
+    for (int a = a0; a < a1; a++) {
         float acc = w[OFF_B1 + a];
         for (int m = 0; m < MLP_IN; m++) acc += w[OFF_W1 + a * MLP_IN + m] * sX[s][m];
         if (acc > 0.0f) mask1 |= 1u << a;
         sH1[s][a] = fmaxf(acc, 0.0f);
     }
-    float z3 = w[OFF_B3];
+    __syncthreads();
 #pragma unroll 4
-    for (int a = 0; a < MLP_H; a++) {
+    for (int a = a0; a < a1; a++) {
         float acc = w[OFF_B2 + a];
         for (int m = 0; m < MLP_H; m++) acc += w[OFF_W2 + a * MLP_H + m] * sH1[s][m];
         if (acc > 0.0f) mask2 |= 1u << a;
-        const float h = fmaxf(acc, 0.0f);
-        sH2[s][a] = h;
-        z3 += w[OFF_W3 + a] * h;
+        sH2[s][a] = fmaxf(acc, 0.0f);
     }
+    __syncthreads();
+    float z3 = w[OFF_B3];
+#pragma unroll
+    for (int a = 0; a < MLP_H; a++) z3 += w[OFF_W3 + a] * sH2[s][a];
     float d3 = 0.0f, loss = 0.0f;
     if (live) {
         const float y = label[src], wt = y > 0.5f ? pos_w : 1.0f;
         loss = wt * (fmaxf(z3, 0.0f) - z3 * y + log1pf(expf(-fabsf(z3))));
         d3 = wt * (1.0f / (1.0f + expf(-z3)) - y);
     }
-    for (int a = 0; a < MLP_H; a++) sD2[s][a] = ((mask2 >> a) & 1u) ? d3 * w[OFF_W3 + a] : 0.0f;
+    for (int a = a0; a < a1; a++) sD2[s][a] = ((mask2 >> a) & 1u) ? d3 * w[OFF_W3 + a] : 0.0f;
+    __syncthreads();
 #pragma unroll 4
-    for (int m = 0; m < MLP_H; m++) {
+    for (int m = a0; m < a1; m++) {
         float acc = 0.0f;
         for (int a = 0; a < MLP_H; a++) acc += w[OFF_W2 + a * MLP_H + m] * sD2[s][a];
         sD1[s][m] = ((mask1 >> m) & 1u) ? acc : 0.0f;
     }
-    sD3[s] = d3; sLoss[s] = loss;
+    if (q == 0) { sD3[s] = d3; sLoss[s] = loss; }
     __syncthreads();
     float *out = part + (long long)blockIdx.x * MLP_NNET;
-    for (int o = s; o < MLP_NNET; o += TB) {
+    for (int o = threadIdx.x; o < MLP_NNET; o += TB * TQ) {
         float acc = 0.0f;
         if (o < MLP_H * MLP_IN) {                       // W1[a][m]
             const int a = o / MLP_IN, m = o % MLP_IN;
@@ -516,39 +525,41 @@ __global__ void __launch_bounds__(TB) k_mlp_grad(const float *__restrict__ w, co
         }
         out[o] = acc;
     }
-    if (s == 0) {
+    if (threadIdx.x == 0) {
         float l = 0.0f;
         for (int q = 0; q < TB; q++) l += sLoss[q];
         lpart[blockIdx.x] = l;
     }
 }
 
-// fixed-order sum over blocks: grad[o] = sum_b part[b][o]; loss likewise
-__global__ void k_mlp_reduce(const float *__restrict__ part, const float *__restrict__ lpart, int nb,
-                             float *__restrict__ grad, double *__restrict__ loss) {
+// Fixed-order sum over blocks: grad[o] = sum_b part[b][o]; loss likewise, by a
+// thread of its own.  With w the Adam step on the network part of the parameter
+// vector follows (grad = batch sum).  The sums are serial chains behind loads
+// that do not depend on them: unrolled, a chain waits for memory once in 32
+// (18 + 3 -> 15 us for 256 blocks, the Adam step included).
+struct AdamStep { float *w, *m1, *m2; float scale, lr, b1, b2, eps, c1, c2; };
+constexpr int RT = 32;     // threads per block
+__global__ void __launch_bounds__(RT) k_mlp_reduce(const float *__restrict__ part, const float *__restrict__ lpart, int nb,
+                                                   float *__restrict__ grad, double *__restrict__ loss, AdamStep s) {
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o < MLP_NNET) {
         float acc = 0.0f;
+#pragma unroll 32
         for (int b = 0; b < nb; b++) acc += part[(long long)b * MLP_NNET + o];
         grad[o] = acc;
+        if (s.w) {
+            const float g = acc * s.scale;
+            const float a = s.b1 * s.m1[o] + (1.0f - s.b1) * g, v = s.b2 * s.m2[o] + (1.0f - s.b2) * g * g;
+            s.m1[o] = a; s.m2[o] = v;
+            s.w[OFF_W1 + o] -= s.lr * (a / s.c1) / (sqrtf(v / s.c2) + s.eps);
+        }
     }
-    if (o == 0) {
+    if (o == MLP_NNET) {
         double l = 0.0;
+#pragma unroll 32
         for (int b = 0; b < nb; b++) l += lpart[b];
         *loss += l;
     }
-}
-
-// Adam on the network part of the parameter vector (grad = batch sum)
-__global__ void k_mlp_adam(float *__restrict__ w, const float *__restrict__ grad, float *__restrict__ m1,
-                           float *__restrict__ m2, float scale, float lr, float b1, float b2, float eps,
-                           float c1, float c2) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= MLP_NNET) return;
-    const float g = grad[o] * scale;
-    const float a = b1 * m1[o] + (1.0f - b1) * g, v = b2 * m2[o] + (1.0f - b2) * g * g;
-    m1[o] = a; m2[o] = v;
-    w[OFF_W1 + o] -= lr * (a / c1) / (sqrtf(v / c2) + eps);
 }
 
 // ---------------------------------------------------------------------------
@@ -626,19 +637,28 @@ cudaError_t launch_mlp_infer(const float *w, const float *feat, long long n, flo
 }
 
 // gradient (batch sum) and loss sum of rows idx[0..n) (or 0..n)
+static void mlp_grad_reduce(const float *w, const float *feat, const float *label, const int *idx, long long n,
+                            float pos_w, float *part, float *lpart, float *grad, double *loss, const AdamStep &step,
+                            cudaStream_t st) {
+    const int nb = mlp_grad_blocks(n);
+    k_mlp_grad<<<nb, TB * TQ, 0, st>>>(w, feat, label, idx, n, pos_w, part, lpart);
+    k_mlp_reduce<<<MLP_NNET / RT + 1, RT, 0, st>>>(part, lpart, nb, grad, loss, step);
+}
+
 cudaError_t launch_mlp_grad(const float *w, const float *feat, const float *label, const int *idx, long long n,
                             float pos_w, float *part, float *lpart, float *grad, double *loss, cudaStream_t st) {
-    const int nb = mlp_grad_blocks(n);
-    k_mlp_grad<<<nb, TB, 0, st>>>(w, feat, label, idx, n, pos_w, part, lpart);
-    k_mlp_reduce<<<(MLP_NNET + 255) / 256, 256, 0, st>>>(part, lpart, nb, grad, loss);
+    mlp_grad_reduce(w, feat, label, idx, n, pos_w, part, lpart, grad, loss, AdamStep{}, st);
     return cudaGetLastError();
 }
 
-cudaError_t launch_mlp_adam(float *w, const float *grad, float *m1, float *m2, float scale, float lr, int t,
+// one Adam step t on the batch's gradient
+cudaError_t launch_mlp_step(float *w, const float *feat, const float *label, const int *idx, long long n, float pos_w,
+                            float *part, float *lpart, float *grad, double *loss, float *m1, float *m2, float lr, int t,
                             cudaStream_t st) {
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.0f - powf(b1, (float)t), c2 = 1.0f - powf(b2, (float)t);
-    k_mlp_adam<<<(MLP_NNET + 255) / 256, 256, 0, st>>>(w, grad, m1, m2, scale, lr, b1, b2, 1e-8f, c1, c2);
+    mlp_grad_reduce(w, feat, label, idx, n, pos_w, part, lpart, grad, loss,
+                    AdamStep{w, m1, m2, 1.0f / (float)n, lr, b1, b2, 1e-8f, c1, c2}, st);
     return cudaGetLastError();
 }
 
