@@ -31,8 +31,8 @@ cudaError_t launch_ghost(const Params &p, double *const *fields, const int *dirm
 cudaError_t launch_ghost32(const Params &p, float *const *fields, const int *dirmask, int nf, cudaStream_t st);
 cudaError_t launch_prims_to_fp32(const Params &p, cudaStream_t st);
 cudaError_t launch_flag_hist(const Params &p, unsigned long long *counts, cudaStream_t st);
-cudaError_t launch_vis_ev(const Params &p, cudaStream_t st);
-cudaError_t launch_vis_div(const Params &p, int krk, int k0, int k1, cudaStream_t st);
+cudaError_t launch_vis_ev(const Params &p, int images, cudaStream_t st);
+cudaError_t launch_vis_div(const Params &p, int krk, int k0, int k1, int images, cudaStream_t st);
 void ev_ghost_fields(const Params &p, void *fields[12], int dirmask[12]);
 cudaError_t launch_rk(const Params &p, int krk, cudaStream_t st);
 cudaError_t launch_rk_only(const Params &p, int krk, cudaStream_t st);
@@ -703,26 +703,27 @@ static int rhs(ocfd_b200_ctx *ctx, int krk, int fused_rk, bool skip_sensor = fal
         int rc = rhs_sensor(ctx);
         if (rc) return rc;
     }
-    {
+    // On one GPU the viscous kernels write the periodic images of what they
+    // form: Ev, and in a whole step the primitives of its first two stages
+    // (the next step's sensor reads the ghosts of the last stage's start;
+    // a boundary-condition family changes values afterwards).
+    const int images = ctx->slab ? 0 : p.periodic[0] | p.periodic[1] << 1 | p.periodic[2] << 2;
+    const bool prim_images = !ctx->slab && !p.ibc;
+    if (!(fused_rk > 1 && prim_images)) {
         TimerScope ts(ctx, T_GHOST);
         int rc = ghost_prims(ctx, true);      // the z planes arrive while the x and y sweeps run
         if (rc) return rc;
     }
-    // On one GPU the viscous fluxes and their ghost fill (they read the
-    // primitives only) go to a second stream beside the inviscid sweeps; the
+    // There the viscous fluxes, which read the primitives only,
+    // go to a second stream beside the inviscid sweeps; the
     // divergence kernel waits for both.  Timed runs keep the families apart.
     const bool side = ctx->vstream && !ctx->slab && !ctx->timing;
-    void *evf[12]; int evmask[12];
-    ocfd::ev_ghost_fields(p, evf, evmask);
     if (side) {
         CK(cudaEventRecord(ctx->vev[0], ctx->stream), "viscous fork");
         CK(cudaStreamWaitEvent(ctx->vstream, ctx->vev[0], 0), "viscous fork");
-        CK(ocfd::launch_vis_ev(p, ctx->vstream), "viscous fluxes");
-        CK(p.mixed ? ghost_launch(p, reinterpret_cast<float *const *>(evf), evmask, 12, ctx->vstream)
-                   : ghost_launch(p, reinterpret_cast<double *const *>(evf), evmask, 12, ctx->vstream),
-           "Ev ghost fill");
+        CK(ocfd::launch_vis_ev(p, images, ctx->vstream), "viscous fluxes");
         CK(cudaEventRecord(ctx->vev[1], ctx->vstream), "viscous join");
-        ctx->launches += 2;
+        ctx->launches += 1;
     }
     {
         TimerScope ts(ctx, T_SWEEP);
@@ -744,17 +745,22 @@ static int rhs(ocfd_b200_ctx *ctx, int krk, int fused_rk, bool skip_sensor = fal
         if (side) {
             CK(cudaStreamWaitEvent(ctx->stream, ctx->vev[1], 0), "viscous join");
         } else {
-            CK(ocfd::launch_vis_ev(p, ctx->stream), "viscous fluxes");
+            CK(ocfd::launch_vis_ev(p, images, ctx->stream), "viscous fluxes");
+            ctx->launches += 1;
             // (forming the planes away from the slab faces while the Ev_z planes
             // travel, and the two bands next to the faces after, measured slower
             // than one launch after the exchange: the small band launches and the
             // extra tail cost more than the exchange they hide)
-            int rc = p.mixed ? fill_ghosts(ctx, reinterpret_cast<float *const *>(evf), evmask, 12, "Ev ghost fill")
-                             : fill_ghosts(ctx, reinterpret_cast<double *const *>(evf), evmask, 12, "Ev ghost fill");
-            if (rc) return rc;
-            ctx->launches += 1;
+            if (ctx->slab) {
+                void *evf[12]; int evmask[12];
+                ocfd::ev_ghost_fields(p, evf, evmask);
+                int rc = p.mixed ? fill_ghosts(ctx, reinterpret_cast<float *const *>(evf), evmask, 12, "Ev ghost fill")
+                                 : fill_ghosts(ctx, reinterpret_cast<double *const *>(evf), evmask, 12, "Ev ghost fill");
+                if (rc) return rc;
+            }
         }
-        CK(ocfd::launch_vis_div(p, fused_rk, 0, p.nz, ctx->stream), "viscous divergence");
+        CK(ocfd::launch_vis_div(p, fused_rk, 0, p.nz, prim_images && fused_rk < 3 ? images : 0, ctx->stream),
+           "viscous divergence");
         ctx->launches += 1;
     }
     if (fused_rk && p.ibc) {        // OCFD_bc: boundary values, then the faces

@@ -227,6 +227,14 @@ __device__ __forceinline__ void cons_to_prim(const Params &p, const double f[5],
     T2 = div_const(f[4] - 0.5 * d1 * (u1 * u1 + v1 * v1 + w1 * w1), dcv, 1.0 / dcv);
 }
 
+// Offset from a cell to its periodic image in the ghosts of a direction (cell
+// X of n, stride s), 0 where it has none.  On one GPU the kernels that form a
+// field write its images as k_ghost would (image bit d for direction d), in
+// place of a launch that reads the slabs back.
+__device__ __forceinline__ long long image(int X, int n, long long s) {
+    return X < OCFD_LAP ? n * s : X >= n - OCFD_LAP ? -n * s : 0;
+}
+
 // Cell of a thread of the viscous kernels: a block of 256 threads covers a
 // 32 x 8 tile of one z plane (grid: x tiles * y tiles, nz), so most y
 // neighbours of its cells are loaded by the same block and meet in L1.
@@ -245,7 +253,7 @@ __device__ __forceinline__ bool tile_cell(const Params &p, int &i, int &j, int &
 // grid directions (uk, ui, us ...) and its metrics m, of k_vis_ev and k_vev.
 // The multiply-adds are spelled out: the two form the same bits.
 template <bool UNI, typename R>
-__device__ __forceinline__ void vis_fluxes(const Params &p, long long o, const R (&m)[3][3], R Amu,
+__device__ __forceinline__ void vis_fluxes(const Params &p, long long o, int images, int i, int j, int k, const R (&m)[3][3], R Amu,
                                            R uk, R ui, R us, R vk, R vi, R vs, R wk, R wi, R ws, R Tk, R Ti, R Ts,
                                            R uu, R vv, R ww) {
     auto dot = [](const R (&a)[3], R x, R y, R z) { return fma(a[0], x, fma(a[1], y, a[2] * z)); };
@@ -268,8 +276,12 @@ __device__ __forceinline__ void vis_fluxes(const Params &p, long long o, const R
         const R a[3] = { m[dd][0] * Aj1, m[dd][1] * Aj1, m[dd][2] * Aj1 };
         R *ev = evb + (long long)(4 * dd) * p.lapN + o;
         const R v[4] = { dot(a, s11, s12, s13), dot(a, s12, s22, s23), dot(a, s13, s23, s33), dot(a, E1, E2, E3) };
+        const long long g = !((images >> dd) & 1) ? 0 : dd == 0 ? image(i, p.nx, 1) : dd == 1 ? image(j, p.ny, p.ys) : image(k, p.nz, p.zs);
 #pragma unroll
-        for (int q = 0; q < 4; q++) ev[q * p.lapN] = v[q];
+        for (int q = 0; q < 4; q++) {
+            ev[q * p.lapN] = v[q];
+            if (g) ev[q * p.lapN + g] = v[q];
+        }
     }
 }
 
@@ -282,7 +294,7 @@ __device__ __forceinline__ void vis_fluxes(const Params &p, long long o, const R
 // registers (4 blocks an SM) hold them.  256^3: 770 -> 592 us (5 blocks 642, 3
 // 624); ramp 512x128x64 367 -> 268 us (5 and 3 blocks 322).
 template <bool UNI, bool BND, bool C8, typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 8 ? 4 : 6) k_vis_ev(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(256, sizeof(R) == 8 ? 4 : 6) k_vis_ev(const __grid_constant__ Params p, int images) {
     int i, j, k;
     long long tid;
     if (!tile_cell(p, i, j, k, tid)) return;
@@ -299,14 +311,14 @@ __global__ void __launch_bounds__(256, sizeof(R) == 8 ? 4 : 6) k_vis_ev(const __
     auto dz = [&](const R *f) { return BND ? d0b<C8>(f, o, p.zs, cz, k, p.nz, p.bnd_lo[2], p.bnd_hi[2]) : d0<C8>(f, o, p.zs, cz); };
     const R uk = dx(U), ui = dy(U), us = dz(U), vk = dx(V), vi = dy(V), vs = dz(V);
     const R wk = dx(W), wi = dy(W), ws = dz(W), Tk = dx(TT), Ti = dy(TT), Ts = dz(TT);
-    vis_fluxes<UNI, R>(p, o, m, Amu, uk, ui, us, vk, vi, vs, wk, wi, ws, Tk, Ti, Ts, U[o], V[o], W[o]);
+    vis_fluxes<UNI, R>(p, o, images, i, j, k, m, Amu, uk, ui, us, vk, vi, vs, wk, wi, ws, Tk, Ti, Ts, U[o], V[o], W[o]);
 }
 
 // RK stage (src/OCFD_time.cu:44-94) + cons_to_pri (src/commen_kernel.cu:77-109)
 // + pri_to_cons re-projection on the six faces (src/OCFD_boundary.cu:40-91)
 // for one cell, given its final du
 // (fn0, fk0: U^n and U^k of the cell, read by the caller)
-__device__ __forceinline__ void rk_cell_pre(const Params &p, int krk, long long tid, int i, int j, int k,
+__device__ __forceinline__ void rk_cell_pre(const Params &p, int krk, int images, long long tid, int i, int j, int k,
                                             const double du[5], const double fn0[5], const double fk0[5]) {
     const long long N = p.N;
     double f[5];
@@ -332,9 +344,24 @@ __device__ __forceinline__ void rk_cell_pre(const Params &p, int krk, long long 
     cons_to_prim(p, f, d1, u1, v1, w1, T2);
     const bool face = (i == 0) || (i == p.nx - 1) || (j == 0) || (j == p.ny - 1) || (k == 0 && p.zface_lo) ||
                       (k == p.nz - 1 && p.zface_hi);
-    if (p.mixed) {      // the stencils of the precision form read FP32 primitives
-        p.prim32[0][o] = (float)d1; p.prim32[1][o] = (float)u1; p.prim32[2][o] = (float)v1;
-        p.prim32[3][o] = (float)w1; p.prim32[4][o] = (float)T2;
+    // the stencils of the precision form read FP32 primitives
+    auto put = [&](long long q) {
+        if (p.mixed) {
+            p.prim32[0][q] = (float)d1; p.prim32[1][q] = (float)u1; p.prim32[2][q] = (float)v1;
+            p.prim32[3][q] = (float)w1; p.prim32[4][q] = (float)T2;
+        } else {
+            p.prim[0][q] = d1; p.prim[1][q] = u1; p.prim[2][q] = v1; p.prim[3][q] = w1; p.prim[4][q] = T2;
+        }
+    };
+    put(o);
+    if (images) {
+        const long long gx = images & 1 ? image(i, p.nx, 1) : 0, gy = images & 2 ? image(j, p.ny, p.ys) : 0;
+        const long long gz = images & 4 ? image(k, p.nz, p.zs) : 0;
+        if (gx) put(o + gx);
+        if (gy) put(o + gy);
+        if (gz) put(o + gz);
+    }
+    if (p.mixed) {
         // the boundary-condition family works on FP64 primitives: its wall
         // law reads the four rows next to the wall and the face re-projection
         // reads the face cells.  With a filter the step's FP64 primitives are
@@ -343,8 +370,6 @@ __device__ __forceinline__ void rk_cell_pre(const Params &p, int krk, long long 
         if ((p.ibc && (face || j <= OCFD_LAP)) || (krk == 3 && p.flap)) {
             p.prim[0][o] = d1; p.prim[1][o] = u1; p.prim[2][o] = v1; p.prim[3][o] = w1; p.prim[4][o] = T2;
         }
-    } else {
-        p.prim[0][o] = d1; p.prim[1][o] = u1; p.prim[2][o] = v1; p.prim[3][o] = w1; p.prim[4][o] = T2;
     }
     // cons_to_pri_kernel also leaves the pressure (src/commen_kernel.cu:107),
     // which the filter after the step reads (FP32 in the precision form)
@@ -365,7 +390,7 @@ __device__ __forceinline__ void rk_cell_pre(const Params &p, int krk, long long 
 #pragma unroll
     for (int m = 0; m < 5; m++) p.f[m * N + tid] = f[m];
 }
-__device__ __forceinline__ void rk_cell(const Params &p, int krk, long long tid, int i, int j, int k,
+__device__ __forceinline__ void rk_cell(const Params &p, int krk, int images, long long tid, int i, int j, int k,
                                         const double du[5]) {
     double fn0[5], fk0[5];
 #pragma unroll
@@ -373,7 +398,7 @@ __device__ __forceinline__ void rk_cell(const Params &p, int krk, long long tid,
         fn0[m] = p.fn[m * p.N + tid];
         fk0[m] = krk == 1 ? 0.0 : p.f[m * p.N + tid];
     }
-    rk_cell_pre(p, krk, tid, i, j, k, du, fn0, fk0);
+    rk_cell_pre(p, krk, images, tid, i, j, k, du, fn0, fk0);
 }
 
 // du[1..4] += Ajac * d(Ev)/d(xi) for x, then y, then z
@@ -385,7 +410,7 @@ __device__ __forceinline__ void rk_cell(const Params &p, int krk, long long tid,
 // 1077 -> 932 us (6 blocks 994, 4 955); with closures 6 blocks (ramp
 // 512x128x64 276 us; 4 324, 3 321).
 template <bool UNI, bool BND, bool C8, bool RK, typename R>
-__global__ void __launch_bounds__(256, BND || sizeof(R) == 4 ? 6 : 3) k_vis_div(const __grid_constant__ Params p, int krk, int k0) {
+__global__ void __launch_bounds__(256, BND || sizeof(R) == 4 ? 6 : 3) k_vis_div(const __grid_constant__ Params p, int krk, int k0, int images) {
     int i, j, k;
     long long tid;
     if (!tile_cell(p, i, j, k, tid, k0)) return;
@@ -414,7 +439,7 @@ __global__ void __launch_bounds__(256, BND || sizeof(R) == 4 ? 6 : 3) k_vis_div(
         double a64[5];
 #pragma unroll
         for (int m = 0; m < 5; m++) a64[m] = (double)acc[m];
-        rk_cell(p, krk, tid, i, j, k, a64);
+        rk_cell(p, krk, images, tid, i, j, k, a64);
     } else {
 #pragma unroll
         for (int m = 0; m < 4; m++) du[(m + 1) * p.N + tid] = acc[m + 1];
@@ -479,7 +504,8 @@ template <bool UNI, typename R, int H>
 // (two blocks per SM: a budget for three spills and measured 14 % slower in FP32)
 __global__ void __launch_bounds__(VX * VY, 2)
 k_vdiv(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tmx,
-       const __grid_constant__ CUtensorMap tmy, const __grid_constant__ CUtensorMap tmz, int krk, int seg_len) {
+       const __grid_constant__ CUtensorMap tmy, const __grid_constant__ CUtensorMap tmz, int krk, int seg_len,
+       int images) {
     using T = VdivTiles<R, H>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ unsigned long long zbar[T::NZS], xybar[2];
@@ -611,7 +637,7 @@ k_vdiv(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tmx
                 double a64[5];
 #pragma unroll
                 for (int m = 0; m < 5; m++) a64[m] = (double)acc[m];
-                rk_cell_pre(p, krk, ci, i, j, k, a64, fn0, fk0);
+                rk_cell_pre(p, krk, images, ci, i, j, k, a64, fn0, fk0);
             }
             // plane k-H's slot and buffer b are free; a wait that ran out
             // anywhere in the block ends the block's work
@@ -653,7 +679,7 @@ struct VevTiles {
 
 template <bool UNI, typename R, int H>
 __global__ void __launch_bounds__(VX * VY, sizeof(R) == 8 ? 1 : 3)
-k_vev(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tmq, int seg_len) {
+k_vev(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tmq, int seg_len, int images) {
     using T = VevTiles<R, H>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ unsigned long long zbar[T::NZS];
@@ -730,7 +756,7 @@ k_vev(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tmq,
                         ds[f] = d0bw<R, H>(vz, cz, k, p.nz, p.bnd_lo[2], p.bnd_hi[2]);
                     }
                 }
-                vis_fluxes<UNI, R>(p, o, m, Amu, dk[0], di[0], ds[0], dk[1], di[1], ds[1], dk[2], di[2], ds[2],
+                vis_fluxes<UNI, R>(p, o, images, i, j, k, m, Amu, dk[0], di[0], ds[0], dk[1], di[1], ds[1], dk[2], di[2], ds[2],
                                    dk[3], di[3], ds[3], at(k, 0, 0, 0), at(k, 1, 0, 0), at(k, 2, 0, 0));
             }
             if (__syncthreads_or(failed)) { failed = true; break; }
@@ -817,7 +843,7 @@ __global__ void k_rk_update(Params p, int krk) {
     double du[5];
 #pragma unroll
     for (int m = 0; m < 5; m++) du[m] = p.mixed ? (double)p.du32[m * p.N + tid] : p.du[m * p.N + tid];
-    rk_cell(p, krk, tid, i, j, k, du);
+    rk_cell(p, krk, 0, tid, i, j, k, du);
 }
 
 // Unfused pieces of the same update for the reference-named per-stage API:
@@ -1046,53 +1072,53 @@ cudaError_t launch_ghost32(const Params &p, float *const *fields, const int *dir
 
 
 template <typename R>
-static cudaError_t launch_vis_ev_t(const Params &p, cudaStream_t st) {
+static cudaError_t launch_vis_ev_t(const Params &p, int images, cudaStream_t st) {
     const dim3 nb((unsigned)(((p.nx + VT_X - 1) / VT_X) * ((p.ny + VT_Y - 1) / VT_Y)), (unsigned)p.nz);
     const bool c8 = p.scheme_vis == 204;
     if (p.has_bnd)
-        c8 ? k_vis_ev<false, true, true, R><<<nb, 256, 0, st>>>(p) : k_vis_ev<false, true, false, R><<<nb, 256, 0, st>>>(p);
+        c8 ? k_vis_ev<false, true, true, R><<<nb, 256, 0, st>>>(p, images) : k_vis_ev<false, true, false, R><<<nb, 256, 0, st>>>(p, images);
     else if (p.uniform_metrics)
-        c8 ? k_vis_ev<true, false, true, R><<<nb, 256, 0, st>>>(p) : k_vis_ev<true, false, false, R><<<nb, 256, 0, st>>>(p);
+        c8 ? k_vis_ev<true, false, true, R><<<nb, 256, 0, st>>>(p, images) : k_vis_ev<true, false, false, R><<<nb, 256, 0, st>>>(p, images);
     else
-        c8 ? k_vis_ev<false, false, true, R><<<nb, 256, 0, st>>>(p) : k_vis_ev<false, false, false, R><<<nb, 256, 0, st>>>(p);
+        c8 ? k_vis_ev<false, false, true, R><<<nb, 256, 0, st>>>(p, images) : k_vis_ev<false, false, false, R><<<nb, 256, 0, st>>>(p, images);
     return cudaGetLastError();
 }
 
 template <bool RK, typename R>
-static cudaError_t launch_vis_div_t(const Params &p, int krk, int k0, int k1, cudaStream_t st) {
+static cudaError_t launch_vis_div_t(const Params &p, int krk, int k0, int k1, int images, cudaStream_t st) {
     if (k1 <= k0) return cudaSuccess;
     const dim3 nb((unsigned)(((p.nx + VT_X - 1) / VT_X) * ((p.ny + VT_Y - 1) / VT_Y)), (unsigned)(k1 - k0));
     const bool c8 = p.scheme_vis == 204;
     if (p.has_bnd)
-        c8 ? k_vis_div<false, true, true, RK, R><<<nb, 256, 0, st>>>(p, krk, k0)
-           : k_vis_div<false, true, false, RK, R><<<nb, 256, 0, st>>>(p, krk, k0);
+        c8 ? k_vis_div<false, true, true, RK, R><<<nb, 256, 0, st>>>(p, krk, k0, images)
+           : k_vis_div<false, true, false, RK, R><<<nb, 256, 0, st>>>(p, krk, k0, images);
     else if (p.uniform_metrics)
-        c8 ? k_vis_div<true, false, true, RK, R><<<nb, 256, 0, st>>>(p, krk, k0)
-           : k_vis_div<true, false, false, RK, R><<<nb, 256, 0, st>>>(p, krk, k0);
+        c8 ? k_vis_div<true, false, true, RK, R><<<nb, 256, 0, st>>>(p, krk, k0, images)
+           : k_vis_div<true, false, false, RK, R><<<nb, 256, 0, st>>>(p, krk, k0, images);
     else
-        c8 ? k_vis_div<false, false, true, RK, R><<<nb, 256, 0, st>>>(p, krk, k0)
-           : k_vis_div<false, false, false, RK, R><<<nb, 256, 0, st>>>(p, krk, k0);
+        c8 ? k_vis_div<false, false, true, RK, R><<<nb, 256, 0, st>>>(p, krk, k0, images)
+           : k_vis_div<false, false, false, RK, R><<<nb, 256, 0, st>>>(p, krk, k0, images);
     return cudaGetLastError();
 }
 
 // The viscous part in two launches with the Ev ghost exchange between them:
 // k_vis_ev forms the 12 Ev fields (4 per direction) on the interior; the
-// caller fills the ghosts of each direction's four (ev_ghost_fields); then
-// k_vis_div.  krk = 0: viscous terms into du; krk = 1..3: viscous terms,
+// caller fills the ghosts of each direction's four (ev_ghost_fields) that
+// images does not leave to the kernel; then k_vis_div, images for the primitives.  krk = 0: viscous terms into du; krk = 1..3: viscous terms,
 // then the RK stage update in the same kernel (du is not written).  FP32
 // stencils in the precision form.
 template <typename R, int H>
-static bool launch_vev_h(const Params &p, cudaStream_t st, cudaError_t &err);
-cudaError_t launch_vis_ev(const Params &p, cudaStream_t st) {
+static bool launch_vev_h(const Params &p, int images, cudaStream_t st, cudaError_t &err);
+cudaError_t launch_vis_ev(const Params &p, int images, cudaStream_t st) {
     const bool staged = p.vis_impl == 2 || (p.vis_impl == 0 && p.mixed);
     if (staged && p.kerr) {
         cudaError_t e = cudaSuccess;
         const bool c8 = p.scheme_vis == 204;
-        const bool done = p.mixed ? (c8 ? launch_vev_h<float, 4>(p, st, e) : launch_vev_h<float, 3>(p, st, e))
-                                  : (c8 ? launch_vev_h<double, 4>(p, st, e) : launch_vev_h<double, 3>(p, st, e));
+        const bool done = p.mixed ? (c8 ? launch_vev_h<float, 4>(p, images, st, e) : launch_vev_h<float, 3>(p, images, st, e))
+                                  : (c8 ? launch_vev_h<double, 4>(p, images, st, e) : launch_vev_h<double, 3>(p, images, st, e));
         if (done) return e;
     }
-    return p.mixed ? launch_vis_ev_t<float>(p, st) : launch_vis_ev_t<double>(p, st);
+    return p.mixed ? launch_vis_ev_t<float>(p, images, st) : launch_vis_ev_t<double>(p, images, st);
 }
 
 // persistent grid of the staged viscous kernels: blocks per SM from their
@@ -1134,7 +1160,7 @@ static void staged_grid(const Params &p, K kern, size_t smem_bytes, unsigned &nb
 
 // the staged Ev kernel; false when the tensor map cannot be formed
 template <typename R, int H>
-static bool launch_vev_h(const Params &p, cudaStream_t st, cudaError_t &err) {
+static bool launch_vev_h(const Params &p, int images, cudaStream_t st, cudaError_t &err) {
     using T = VevTiles<R, H>;
     const unsigned long long eb = sizeof(R);
     const unsigned long long dims[4] = { (unsigned long long)p.ys, (unsigned long long)(p.ny + 2 * OCFD_LAP),
@@ -1151,7 +1177,7 @@ static bool launch_vev_h(const Params &p, cudaStream_t st, cudaError_t &err) {
     int seg;
     auto kern = p.uniform_metrics ? k_vev<true, R, H> : k_vev<false, R, H>;
     staged_grid(p, kern, T::bytes, nb, seg);
-    kern<<<nb, VX * VY, T::bytes, st>>>(p, tmq, seg);
+    kern<<<nb, VX * VY, T::bytes, st>>>(p, tmq, seg, images);
     err = cudaGetLastError();
     return true;
 }
@@ -1159,7 +1185,7 @@ static bool launch_vev_h(const Params &p, cudaStream_t st, cudaError_t &err) {
 // the staged divergence + RK stage over the whole slab; false when the tensor
 // maps cannot be formed (the caller then uses k_vis_div)
 template <typename R, int H>
-static bool launch_vdiv_h(const Params &p, int krk, cudaStream_t st, cudaError_t &err) {
+static bool launch_vdiv_h(const Params &p, int krk, int images, cudaStream_t st, cudaError_t &err) {
     using T = VdivTiles<R, H>;
     const unsigned long long eb = sizeof(R);
     const unsigned long long dims[4] = { (unsigned long long)p.ys, (unsigned long long)(p.ny + 2 * OCFD_LAP),
@@ -1177,7 +1203,7 @@ static bool launch_vdiv_h(const Params &p, int krk, cudaStream_t st, cudaError_t
     int best;
     auto kern = p.uniform_metrics ? k_vdiv<true, R, H> : k_vdiv<false, R, H>;
     staged_grid(p, kern, T::bytes, nb, best);
-    kern<<<nb, VX * VY, T::bytes, st>>>(p, tmx, tmy, tmz, krk, best);
+    kern<<<nb, VX * VY, T::bytes, st>>>(p, tmx, tmy, tmz, krk, best, images);
     err = cudaGetLastError();
     return true;
 }
@@ -1201,18 +1227,18 @@ cudaError_t vdiv_prepare() {
 }
 
 // planes k0 .. k1-1 (the whole slab: 0, nz)
-cudaError_t launch_vis_div(const Params &p, int krk, int k0, int k1, cudaStream_t st) {
+cudaError_t launch_vis_div(const Params &p, int krk, int k0, int k1, int images, cudaStream_t st) {
     const bool staged = p.vis_impl == 2 || (p.vis_impl == 0 && p.mixed);
     if (krk > 0 && k0 == 0 && k1 == p.nz && staged && p.kerr) {
         cudaError_t e = cudaSuccess;
         const bool c8 = p.scheme_vis == 204;
-        const bool done = p.mixed ? (c8 ? launch_vdiv_h<float, 4>(p, krk, st, e) : launch_vdiv_h<float, 3>(p, krk, st, e))
-                                  : (c8 ? launch_vdiv_h<double, 4>(p, krk, st, e) : launch_vdiv_h<double, 3>(p, krk, st, e));
+        const bool done = p.mixed ? (c8 ? launch_vdiv_h<float, 4>(p, krk, images, st, e) : launch_vdiv_h<float, 3>(p, krk, images, st, e))
+                                  : (c8 ? launch_vdiv_h<double, 4>(p, krk, images, st, e) : launch_vdiv_h<double, 3>(p, krk, images, st, e));
         if (done) return e;
     }
     if (krk == 0)
-        return p.mixed ? launch_vis_div_t<false, float>(p, 0, k0, k1, st) : launch_vis_div_t<false, double>(p, 0, k0, k1, st);
-    return p.mixed ? launch_vis_div_t<true, float>(p, krk, k0, k1, st) : launch_vis_div_t<true, double>(p, krk, k0, k1, st);
+        return p.mixed ? launch_vis_div_t<false, float>(p, 0, k0, k1, 0, st) : launch_vis_div_t<false, double>(p, 0, k0, k1, 0, st);
+    return p.mixed ? launch_vis_div_t<true, float>(p, krk, k0, k1, images, st) : launch_vis_div_t<true, double>(p, krk, k0, k1, images, st);
 }
 
 // base pointers of the 12 Ev fields (FP64, or FP32 in the precision form)
