@@ -192,8 +192,8 @@ int ocfd_b200_set_walk_threshold(ocfd_b200_ctx *ctx, double frac);
  * Ev tiles of each plane (x and y with their halos, z in a ring of planes)
  * in shared memory by bulk tensor copies while the block marches along z;
  * 1 reads every Ev value through the L1/L2 caches; 0 (default) the staged
- * kernel in the precision form and the cached one in FP64, each the faster
- * of the two there.  The same arithmetic (results equal bit for bit).  No reference counterpart
+ * kernel in the precision form on grids of a million cells or more without
+ * closed faces and the cached one elsewhere, each the faster of the two there.  The same arithmetic (results equal bit for bit).  No reference counterpart
  * (du_viscous_Jacobian3d_*_final, src/OCFD_NS_Jacobian3d.cu:80-440, is the
  * computation both replace). */
 int ocfd_b200_set_viscous_impl(ocfd_b200_ctx *ctx, int impl);

@@ -1101,6 +1101,17 @@ static cudaError_t launch_vis_div_t(const Params &p, int krk, int k0, int k1, in
     return cudaGetLastError();
 }
 
+// Whether the staged pair runs: asked for, or by default in FP32 on large
+// grids without closures (256^3: divergence 597 us against 627 to 720 cached,
+// fluxes 390 against 397; four steps of 128^3 3.65 against 3.72 ms).  With
+// closures parting a cell's loads the cached pair is the faster (ramp
+// 251x67x45: fluxes 45 us against 60, divergence 48 against 85), and on small
+// grids, where a block's march along z is a serial chain (four steps of 24^3
+// 0.63 against 0.83 ms, 64^3 1.00 against 1.07, level at 96^3).
+static bool vis_staged(const Params &p) {
+    return p.vis_impl == 2 || (p.vis_impl == 0 && p.mixed && !p.has_bnd && p.N >= 1000000);
+}
+
 // The viscous part in two launches with the Ev ghost exchange between them:
 // k_vis_ev forms the 12 Ev fields (4 per direction) on the interior; the
 // caller fills the ghosts of each direction's four (ev_ghost_fields) that
@@ -1110,7 +1121,7 @@ static cudaError_t launch_vis_div_t(const Params &p, int krk, int k0, int k1, in
 template <typename R, int H>
 static bool launch_vev_h(const Params &p, int images, cudaStream_t st, cudaError_t &err);
 cudaError_t launch_vis_ev(const Params &p, int images, cudaStream_t st) {
-    const bool staged = p.vis_impl == 2 || (p.vis_impl == 0 && p.mixed);
+    const bool staged = vis_staged(p);
     if (staged && p.kerr) {
         cudaError_t e = cudaSuccess;
         const bool c8 = p.scheme_vis == 204;
@@ -1228,7 +1239,7 @@ cudaError_t vdiv_prepare() {
 
 // planes k0 .. k1-1 (the whole slab: 0, nz)
 cudaError_t launch_vis_div(const Params &p, int krk, int k0, int k1, int images, cudaStream_t st) {
-    const bool staged = p.vis_impl == 2 || (p.vis_impl == 0 && p.mixed);
+    const bool staged = vis_staged(p);
     if (krk > 0 && k0 == 0 && k1 == p.nz && staged && p.kerr) {
         cudaError_t e = cudaSuccess;
         const bool c8 = p.scheme_vis == 204;
