@@ -928,37 +928,38 @@ __global__ void __launch_bounds__(256) k_load_state(Params p, const double *__re
     const int ntx = (int)((p.ys + 31) / 32), nyl = p.ny + 2 * OCFD_LAP;
     const int il = (int)(blockIdx.x % ntx) * 32 + (int)(threadIdx.x % 32);
     const int jl = (int)(blockIdx.x / ntx) * 8 + (int)(threadIdx.x / 32);
-    const int kl = (int)blockIdx.y;
     if (il >= p.ys || jl >= nyl) return;
-    const long long o = OCFD_IDX(p, (long long)il + p.ys * jl + p.zs * kl, p.lapN), N = p.N;
-    int i = il - OCFD_LAP, j = jl - OCFD_LAP, k = kl - OCFD_LAP;
-    const bool gx = i < 0 || i >= p.nx, gy = j < 0 || j >= p.ny, gz = k < 0 || k >= p.nz;
-    double q[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    const bool ghost = wrap && i < p.nx + OCFD_LAP && (int)gx + (int)gy + (int)gz == 1 &&
-                       ((gx && p.periodic[0]) || (gy && p.periodic[1]) || (gz && p.periodic[2]));
-    const bool inner = !gx && !gy && !gz;
-    if (inner || ghost) {
-        i += i < 0 ? p.nx : i >= p.nx ? -p.nx : 0;
-        j += j < 0 ? p.ny : j >= p.ny ? -p.ny : 0;
-        k += k < 0 ? p.nz : k >= p.nz ? -p.nz : 0;
-        const long long c = in_index(p, i, j, k);
+    for (int kl = (int)blockIdx.y; kl < p.nz + 2 * OCFD_LAP; kl += (int)gridDim.y) {
+        const long long o = OCFD_IDX(p, (long long)il + p.ys * jl + p.zs * kl, p.lapN), N = p.N;
+        int i = il - OCFD_LAP, j = jl - OCFD_LAP, k = kl - OCFD_LAP;
+        const bool gx = i < 0 || i >= p.nx, gy = j < 0 || j >= p.ny, gz = k < 0 || k >= p.nz;
+        double q[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        const bool ghost = wrap && i < p.nx + OCFD_LAP && (int)gx + (int)gy + (int)gz == 1 &&
+                           ((gx && p.periodic[0]) || (gy && p.periodic[1]) || (gz && p.periodic[2]));
+        const bool inner = !gx && !gy && !gz;
+        if (inner || ghost) {
+            i += i < 0 ? p.nx : i >= p.nx ? -p.nx : 0;
+            j += j < 0 ? p.ny : j >= p.ny ? -p.ny : 0;
+            k += k < 0 ? p.nz : k >= p.nz ? -p.nz : 0;
+            const long long c = in_index(p, i, j, k);
 #pragma unroll
-        for (int m = 0; m < 5; m++) q[m] = src[m * N + c];
-        if (inner) {
-            const double d = q[0], u = q[1], v = q[2], w = q[3], T = q[4];
-            p.f[c] = d;
-            p.f[N + c] = u * d;
-            p.f[2 * N + c] = v * d;
-            p.f[3 * N + c] = w * d;
-            p.f[4 * N + c] = d * ((u * u + v * v + w * w) * 0.5 + p.Cv * T);
+            for (int m = 0; m < 5; m++) q[m] = src[m * N + c];
+            if (inner) {
+                const double d = q[0], u = q[1], v = q[2], w = q[3], T = q[4];
+                p.f[c] = d;
+                p.f[N + c] = u * d;
+                p.f[2 * N + c] = v * d;
+                p.f[3 * N + c] = w * d;
+                p.f[4 * N + c] = d * ((u * u + v * v + w * w) * 0.5 + p.Cv * T);
 #pragma unroll
-            for (int m = 0; m < 5; m++) { p.fn[m * N + c] = 0.0; p.du[m * N + c] = 0.0; }
+                for (int m = 0; m < 5; m++) { p.fn[m * N + c] = 0.0; p.du[m * N + c] = 0.0; }
+            }
         }
-    }
 #pragma unroll
-    for (int m = 0; m < 5; m++) {
-        p.prim[m][o] = q[m];
-        if (f32) p.prim32[m][o] = (float)q[m];
+        for (int m = 0; m < 5; m++) {
+            p.prim[m][o] = q[m];
+            if (f32) p.prim32[m][o] = (float)q[m];
+        }
     }
 }
 
@@ -969,22 +970,23 @@ __global__ void __launch_bounds__(256) k_store_state(Params p, double *__restric
     const int ntx = (p.nx + 31) / 32;
     const int i = (int)(blockIdx.x % ntx) * 32 + (int)(threadIdx.x % 32);
     const int j = (int)(blockIdx.x / ntx) * 8 + (int)(threadIdx.x / 32);
-    const int k = (int)blockIdx.y;
     if (i >= p.nx || j >= p.ny) return;
-    const long long o = lap_index(p, i + OCFD_LAP, j + OCFD_LAP, k + OCFD_LAP), c = in_index(p, i, j, k), N = p.N;
-    double q[5];
-    if (from_f) {
-        const double f[5] = {p.f[c], p.f[N + c], p.f[2 * N + c], p.f[3 * N + c], p.f[4 * N + c]};
-        cons_to_prim(p, f, q[0], q[1], q[2], q[3], q[4]);
+    for (int k = (int)blockIdx.y; k < p.nz; k += (int)gridDim.y) {
+        const long long o = lap_index(p, i + OCFD_LAP, j + OCFD_LAP, k + OCFD_LAP), c = in_index(p, i, j, k), N = p.N;
+        double q[5];
+        if (from_f) {
+            const double f[5] = {p.f[c], p.f[N + c], p.f[2 * N + c], p.f[3 * N + c], p.f[4 * N + c]};
+            cons_to_prim(p, f, q[0], q[1], q[2], q[3], q[4]);
 #pragma unroll
-        for (int m = 0; m < 5; m++) p.prim[m][o] = q[m];
-        if (p.pfil) p.pfil[o] = q[4] * q[0] / (p.Gamma * p.Ama * p.Ama);
-    } else {
+            for (int m = 0; m < 5; m++) p.prim[m][o] = q[m];
+            if (p.pfil) p.pfil[o] = q[4] * q[0] / (p.Gamma * p.Ama * p.Ama);
+        } else {
 #pragma unroll
-        for (int m = 0; m < 5; m++) q[m] = p.prim[m][o];
+            for (int m = 0; m < 5; m++) q[m] = p.prim[m][o];
+        }
+#pragma unroll
+        for (int m = 0; m < 5; m++) out[m * N + c] = q[m];
     }
-#pragma unroll
-    for (int m = 0; m < 5; m++) out[m * N + c] = q[m];
 }
 
 // the FP32 primitives of the precision form from the FP64 ones (whole LAP box)
@@ -1281,14 +1283,18 @@ cudaError_t launch_rk(const Params &p, int krk, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+// z extent of a launch over planes, which its blocks stride over: a grid's y
+// dimension ends at 65535 blocks, a state's z dimension and its ghosts need not
+static unsigned grid_planes(int n) { return (unsigned)(n < 65535 ? n : 65535); }
+
 cudaError_t launch_load_state(const Params &p, const double *src, bool wrap, bool f32, cudaStream_t st) {
-    const dim3 grid((unsigned)((p.ys + 31) / 32 * ((p.ny + 2 * OCFD_LAP + 7) / 8)), (unsigned)(p.nz + 2 * OCFD_LAP));
+    const dim3 grid((unsigned)((p.ys + 31) / 32 * ((p.ny + 2 * OCFD_LAP + 7) / 8)), grid_planes(p.nz + 2 * OCFD_LAP));
     k_load_state<<<grid, 256, 0, st>>>(p, src, wrap ? 1 : 0, f32 ? 1 : 0);
     return cudaGetLastError();
 }
 
 cudaError_t launch_store_state(const Params &p, double *out, bool from_f, cudaStream_t st) {
-    const dim3 grid((unsigned)((p.nx + 31) / 32 * ((p.ny + 7) / 8)), (unsigned)p.nz);
+    const dim3 grid((unsigned)((p.nx + 31) / 32 * ((p.ny + 7) / 8)), grid_planes(p.nz));
     k_store_state<<<grid, 256, 0, st>>>(p, out, from_f ? 1 : 0);
     return cudaGetLastError();
 }

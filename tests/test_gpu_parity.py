@@ -486,3 +486,24 @@ def test_every_scheme_in_line(gpu_lib, scheme, char, bounds, dims):
     ua, ub = a.conserved(), b.conserved()
     assert np.all(np.isfinite(ub))
     assert np.all(rel_l2(ua, ub) <= 1e-12), rel_l2(ua, ub)
+
+
+@pytest.mark.parametrize("nz", [65530, 65600])
+def test_state_taller_than_a_launch_grid(gpu_lib, nz):
+    """A state whose planes, or planes and ghosts, are more than the 65535
+    blocks of a launch's second dimension: loaded and read back whole; where
+    a stage's kernels take its planes, advanced by a step."""
+    case = cases.taylor_green(8, seed=2)
+    q = np.stack([np.resize(f, (nz, 8, 8)) + 1e-3 * np.cos(np.arange(nz))[:, None, None] for f in case.prims])
+    case.cfg.nz = nz
+    s = lib.Solver(case.cfg, q, [np.resize(m, (nz, 8, 8)) for m in case.metrics])
+    assert np.array_equal(s.primitives(), q)
+    u = s.conserved()
+    assert np.array_equal(u[0], q[0]) and np.array_equal(u[3], q[3] * q[0])
+    if nz <= 65535:
+        case.cfg.dt = 1e-7
+        a = lib.Solver(case.cfg, q, [np.resize(m, (nz, 8, 8)) for m in case.metrics])
+        a.step(1)
+        p = a.primitives()
+        assert np.all(np.isfinite(p)) and np.array_equal(a.conserved()[0], p[0])
+        assert 0 < np.max(np.abs(p - q)) < 1e-2
