@@ -292,7 +292,9 @@ __device__ __forceinline__ R weno5_core(const R *v, int mask = 7) {
     } else {
         a0 = k0 / b0; a1 = k1 / b1; a2 = k2 / b2;
     }
-    const R q0 = fma((R)3.0, d3, -e3), q1 = fma((R)2.0, d3, d2), q2 = fma((R)2.0, e1, (R)3.0 * d2);
+    // (nor in the sum: beside a closed face its points are ghosts, whose values must not reach the face)
+    const R q0 = mask & 1 ? fma((R)3.0, d3, -e3) : (R)0.0, q1 = mask & 2 ? fma((R)2.0, d3, d2) : (R)0.0;
+    const R q2 = mask & 4 ? fma((R)2.0, e1, (R)3.0 * d2) : (R)0.0;
     return v[3] + fma(a0, q0, fma(a1, q1, a2 * q2)) / ((R)6.0 * (a0 + a1 + a2));
 }
 __device__ __forceinline__ double weno5_p(const double *s) { return weno5_core(s); }
