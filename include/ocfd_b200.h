@@ -106,12 +106,14 @@ int ocfd_b200_uniform_metrics(const ocfd_b200_ctx *ctx);
  * values in shared memory and forms every face, closure and line-end rule
  * in the walk; UP7, and a hybrid direction whose sensor pass marked almost
  * every face UP7 (the choice is read back once per step, after the sensor),
- * take the UP7 walk: rows of four cells a lane in x, per-lane marches in y and
- * z, the few cells beside other faces finished by a second kernel.
+ * take the UP7 walk: rows of four cells a lane in x, in y and z per-lane
+ * marches, or on small grids and rows that leave a march's lanes idle the
+ * ring, the few cells beside other faces finished by a second kernel.
  * 5: the generic walk, every face through one in-loop dispatch (variant 4
  * where projection is asked of a scheme that has none);
  * 6: the in-line walk alone (characteristic hybrid scheme and WENO7 only);
- * 7: as 4 with the y and z UP7 walks through the shared-memory ring; 8: as 4.
+ * 7: as 4 with the y and z UP7 walks through the shared-memory ring; 8: as 4
+ * with those walks as marches.
  * All agree to the parity bound (WENO weights amplify the different multiply-add
  * contractions); 4, 7 and 8 agree bit for bit.  Other values: OCFD_ERR_ARG. */
 int ocfd_b200_set_sweep_impl(ocfd_b200_ctx *ctx, int impl);

@@ -23,6 +23,7 @@ cudaError_t launch_sensor(const Params &p, cudaStream_t st);
 cudaError_t launch_q_criterion(const Params &p, double *q, cudaStream_t st);
 cudaError_t launch_time_average(const Params &p, double *mean5, int n, cudaStream_t st);
 bool march_supported(const Params &p, int dir);
+bool march_is_faster(const Params &p);
 cudaError_t march_prepare();
 cudaError_t row_prepare();
 cudaError_t vdiv_prepare();
@@ -146,13 +147,14 @@ struct ocfd_b200_ctx {
     float sw_conf_logit = 0.0f;
     int walk4[3] = {1, 1, 1};
     double walk4_threshold = 0.002;     // deferred cells per cell above which the inline walk is used
-    // the UP7 walk of the y and z sweeps as per-lane marches (ocfd_march.cu);
-    // 0: the shared-memory ring walk there too (sweep variant 7)
     bool vdiv_ok = true;        // the staged divergence kernel can be launched
     // running time averages of d, u, v, w, T (5 interior fields, allocated on
     // first use) and the number of samples in them
     double *avg_buf = nullptr;
     int avg_n = 0;
+    // the UP7 walk of the y and z sweeps: 1 per-lane marches (ocfd_march.cu) or
+    // the shared-memory ring by march_is_faster, 0 the ring (sweep variant 7),
+    // 2 the marches (variant 8)
     int march = 1;
     // the grid split in z across GPUs: this rank's slab starts at global
     // plane z_offset of nz_global; ghost planes in z come from the
@@ -652,7 +654,8 @@ static int sweeps_auto(ocfd_b200_ctx *ctx) {
         if (w[d]) {
             CK(ocfd::launch_sweep4_dir(p, d, ctx->stream), "inviscid sweeps");
             ctx->launches += 1;
-        } else if (d > 0 && ctx->march && ocfd::march_supported(p, d)) {
+        } else if (d > 0 && ctx->march && ocfd::march_supported(p, d) &&
+                   (ctx->march == 2 || ocfd::march_is_faster(p))) {
             CK(ocfd::launch_march_dir(p, d, ctx->stream), "inviscid sweeps");
             ctx->launches += 2;
         } else {
@@ -1152,7 +1155,7 @@ extern "C" int ocfd_b200_set_walk_threshold(ocfd_b200_ctx *ctx, double frac) {
 
 extern "C" int ocfd_b200_set_sweep_impl(ocfd_b200_ctx *ctx, int impl) {
     if (!ctx || impl < 4 || impl > 8) return OCFD_ERR_ARG;
-    ctx->march = impl == 7 ? 0 : 1;
+    ctx->march = impl == 7 ? 0 : (impl == 8 ? 2 : 1);
     ctx->p.sweep_impl = impl >= 7 ? 4 : impl;
     return OCFD_OK;
 }

@@ -303,6 +303,10 @@ bool march_supported(const Params &p, int dir) {
     return (dir == 1 || dir == 2) && fast_scheme && p.defer[0] != nullptr;
 }
 
+bool march_is_faster(const Params &p) {
+    return walk::march_is_faster(p.nx, p.N, p.uniform_metrics != 0, p.mixed != 0);
+}
+
 // one direction: the march, then the fix-up of its deferred cells (the
 // caller clears the deferred counters once per stage, as for the ring walk)
 cudaError_t launch_march_dir(const Params &p, int dir, cudaStream_t st) {

@@ -203,6 +203,25 @@ inline int segment_cells(long long groups, int n, int LY, long long slots, int s
     return len;
 }
 
+// Which UP7 walk a y or z sweep takes: the marches (ocfd_march.cu; a lane a
+// column of a line, 32 neighbours a warp) or the ring (k_sweep3; 8 columns a
+// warp).  The two form the same bits.  A march is the fewer operations but one
+// serial chain a lane, and the lanes past a row's end idle: it is faster from
+// the size on at which its warps fill the chip, where most of a warp's lanes
+// have a column.  Whole steps, march / ring, us.  FP64, uniform metrics: 56^3
+// 251 / 240, 60^3 270 / 273, 64^3 309 / 321, 96^3 668 / 737; metric fields: 64^3
+// 297 / 288, 96x60x60 418 / 411, 160x33x65 between walls 1901 / 1946, 64x80x80
+// 404 / 446, 12^3 between walls 265 / 212.  FP32: 80^3
+// 385 / 368, 88^3 430 / 433, 96^3 488 / 503.  By the share of lanes with a column:
+// FP64 0.73 (70x300x200) 3224 / 3068, 0.75 (72x256x256) 3367 / 3249, 0.78
+// (100x200x150) 2133 / 2135, 0.83 (80x200x200) 2168 / 2175; FP32 0.81
+// (104x150x150) 1181 / 1164, 0.83 (80x200x200) 1561 / 1536, 0.88 (112^3) 708 / 724.
+inline bool march_is_faster(int nx, long long cells, bool uniform, bool fp32) {
+    const long long lanes = (nx + 31LL) / 32 * 32;
+    if (fp32) return 20LL * nx >= 17 * lanes && cells >= 600000;
+    return 5LL * nx >= 4 * lanes && cells >= (uniform ? 210000 : 300000);
+}
+
 template <int DIR> struct Shape;
 template <> struct Shape<0> { static constexpr int LC = 1, RING = 64; };
 template <> struct Shape<1> { static constexpr int LC = 8, RING = 16; };

@@ -45,7 +45,7 @@ def _extra():
     """(name, case, settings, steps) beyond the golden cases."""
     out = []
     iso = cases.isotropic_turbulence(24, seed=41, charteric=1, hy_dp_intv=(0.002, 0.02))
-    out.append(("iso24_fp32_march_staged", iso, {"precision": 1}, 3))
+    out.append(("iso24_fp32_march_staged", iso, {"precision": 1, "sweep": 8, "viscous": 2}, 3))
     out.append(("iso24_fp32_switch", iso, {"precision": 1, "switch": True}, 3))
     out.append(("iso24_fp64_march_staged", iso, {"sweep": 8, "viscous": 2}, 3))
     out.append(("iso24_fp64_inline", iso, {"sweep": 6}, 2))

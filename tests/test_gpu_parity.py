@@ -245,8 +245,8 @@ def _march_cases():
 
 @pytest.mark.parametrize("name,case", _march_cases(), ids=[n for n, _ in _march_cases()])
 def test_march_matches_ring_walk(name, case, gpu_lib):
-    """The y and z UP7 walks run as per-lane marches (variants 4 and 8) or
-    through the shared-memory ring (variant 7).  Same face and cell arithmetic and the same deferred
+    """The y and z UP7 walks run as per-lane marches (variant 8) or through the
+    shared-memory ring (variant 7), variant 4 whichever is the faster.  Same face and cell arithmetic and the same deferred
     cells, so the same state to the last bit, in FP64 and in the precision
     form; and the FP64 state matches the in-loop dispatch (variant 5) to the
     walk-equivalence bound."""

@@ -1,0 +1,49 @@
+"""The host-side rules that choose and split the inviscid walks
+(ocfd_walk.cuh), compiled for the host: at the sizes where both sides were
+measured they take the faster one."""
+import ctypes
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "opencfd-scu_b200", "csrc")
+
+HOST = r"""
+#include <cmath>
+#define __device__
+#define __forceinline__ inline
+#define __noinline__
+#define __ldg(x) (*(x))
+using std::fma; using std::fabs; using std::sqrt; using std::fmin; using std::fmax;
+#include "ocfd_walk.cuh"
+extern "C" int march(int nx, long long cells, int uniform, int fp32) {
+    return ocfd::walk::march_is_faster(nx, cells, uniform, fp32);
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    d = tmp_path_factory.mktemp("rules")
+    (d / "host.cpp").write_text(HOST)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-shared", "-fPIC", "-I", CSRC, str(d / "host.cpp"),
+                    "-o", str(d / "host.so")], check=True)
+    h = ctypes.CDLL(str(d / "host.so"))
+    h.march.argtypes = [ctypes.c_int, ctypes.c_longlong, ctypes.c_int, ctypes.c_int]
+    return h
+
+
+# (grid, FP64 uniform, FP64 metric fields, FP32): 1 where the marches measured faster, 0 the ring
+MARCH = [((12, 12, 12), 0, 0, 0), ((32, 32, 32), 0, 0, 0), ((48, 48, 48), 0, 0, 0), ((56, 56, 56), 0, 0, 0),
+         ((64, 64, 64), 1, 0, 0), ((65, 64, 64), 0, 0, 0), ((33, 90, 70), 0, 0, 0), ((33, 200, 200), 0, 0, 0),
+         ((70, 120, 100), 0, 0, 0), ((72, 256, 256), 0, 0, 0), ((64, 80, 80), 1, 1, 0), ((84, 84, 84), 1, 1, 0),
+         ((96, 96, 96), 1, 1, 1), ((112, 112, 112), 1, 1, 1), ((256, 256, 256), 1, 1, 1)]
+
+
+@pytest.mark.parametrize("dims,uniform,fields,fp32", MARCH)
+def test_up7_walk_choice(host, dims, uniform, fields, fp32):
+    n = dims[0] * dims[1] * dims[2]
+    assert (host.march(dims[0], n, 1, 0), host.march(dims[0], n, 0, 0), host.march(dims[0], n, 1, 1)) == \
+        (uniform, fields, fp32)
