@@ -540,7 +540,7 @@ cudaError_t launch_dir4(const Params &p, cudaStream_t st) {
     const int n = DIR == 0 ? p.nx : (DIR == 1 ? p.ny : p.nz);
     const long long ngx = (p.nx + LC - 1) / LC;
     const long long groups = DIR == 0 ? ((long long)p.ny * p.nz + LC - 1) / LC : ngx * (DIR == 1 ? p.nz : p.ny);
-    const int seg_len = segment_cells(groups, n, LY, 148LL * MINB * SW, 3);
+    const int seg_len = segment_cells(groups, n, LY, 148LL * MINB * SW, 3, segment_tail<R>());
     dim3 grid((unsigned)((groups + SW - 1) / SW), (unsigned)((n + seg_len - 1) / seg_len));
     constexpr int smem = SW * 10 * (Shape4<DIR, KIND>::RING + LY + 1) * LC * (int)sizeof(R);
     static_assert(smem <= 48 * 1024, "no attribute needed");

@@ -186,8 +186,13 @@ constexpr int SW = 4;          // warps per block
 // the least time: full rounds of resident warps, then one that is part empty
 // and runs no faster than a pass's latency.  One 16^3 step 179 -> 94 us and five
 // 64^3 steps 2.27 -> 2.03 ms against four waves of warps or segments of four
-// passes.
-inline int segment_cells(long long groups, int n, int LY, long long slots, int sat) {
+// passes.  tail: passes of a warp that the launch's slowest warps, those with
+// the most faces that are not the common one, run on alone; long segments make
+// that long too.  Two in FP32, whose pipe three warps do not fill: without it one
+// step of the precision form's WENO7 takes 755 us for 640 (160x33x65 between
+// walls), 1084 for 833 (400x40x40), its hybrid scheme 3280 for 2960 (160^3);
+// over 100 grids of 16^3 to 176^3 5 % less, 3.6 % more at most (50x60x130).
+inline int segment_cells(long long groups, int n, int LY, long long slots, int sat, int tail) {
     long long best = -1;
     int len = n;
     for (int nseg = 1; nseg <= n; nseg++) {
@@ -196,7 +201,7 @@ inline int segment_cells(long long groups, int n, int LY, long long slots, int s
         const long long warps = (groups + SW - 1) / SW * SW * ((n + L - 1) / L), rem = warps % slots;
         const long long full = slots / (4 * 148) > sat ? slots / (4 * 148) : sat;
         const long long part = (rem + 4 * 148 - 1) / (4 * 148);
-        const long long t = P2 * (warps / slots * full + (rem ? (part > sat ? part : sat) : 0));
+        const long long t = P2 * (warps / slots * full + (rem ? (part > sat ? part : sat) : 0) + tail);
         if (best < 0 || t < best) { best = t; len = L; }
         if (P2 == 3) break;             // one pass
     }
@@ -221,6 +226,8 @@ inline bool march_is_faster(int nx, long long cells, bool uniform, bool fp32) {
     if (fp32) return 20LL * nx >= 17 * lanes && cells >= 600000;
     return 5LL * nx >= 4 * lanes && cells >= (uniform ? 210000 : 300000);
 }
+
+template <typename R> constexpr int segment_tail() { return sizeof(R) == 8 ? 0 : 2; }
 
 template <int DIR> struct Shape;
 template <> struct Shape<0> { static constexpr int LC = 1, RING = 64; };

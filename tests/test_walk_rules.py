@@ -21,6 +21,10 @@ using std::fma; using std::fabs; using std::sqrt; using std::fmin; using std::fm
 extern "C" int march(int nx, long long cells, int uniform, int fp32) {
     return ocfd::walk::march_is_faster(nx, cells, uniform, fp32);
 }
+extern "C" int segment(long long groups, int n, int LY, long long slots, int fp32) {
+    using namespace ocfd::walk;
+    return segment_cells(groups, n, LY, slots, 3, fp32 ? segment_tail<float>() : segment_tail<double>());
+}
 """
 
 
@@ -31,6 +35,7 @@ def host(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-shared", "-fPIC", "-I", CSRC, str(d / "host.cpp"),
                     "-o", str(d / "host.so")], check=True)
     h = ctypes.CDLL(str(d / "host.so"))
+    h.segment.argtypes = [ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_int]
     h.march.argtypes = [ctypes.c_int, ctypes.c_longlong, ctypes.c_int, ctypes.c_int]
     return h
 
@@ -47,3 +52,17 @@ def test_up7_walk_choice(host, dims, uniform, fields, fp32):
     n = dims[0] * dims[1] * dims[2]
     assert (host.march(dims[0], n, 1, 0), host.march(dims[0], n, 0, 0), host.march(dims[0], n, 1, 1)) == \
         (uniform, fields, fp32)
+
+
+def test_segments_of_fp32_lines(host):
+    """WENO7 lines in FP32 take more segments than in FP64 where one round of
+    warps would walk long ones beside idle schedulers (both measured, see
+    segment_cells): the z lines of 160x33x65 and the x lines of 400x40x40,
+    five blocks an SM.  Every line is covered whatever the size."""
+    slots = 148 * 5 * 4
+    assert (host.segment(20 * 33, 65, 4, slots, 1), host.segment(20 * 33, 65, 4, slots, 0)) == (11, 22)
+    assert (host.segment(1600, 400, 32, slots, 1), host.segment(1600, 400, 32, slots, 0)) == (58, 400)
+    for n in (8, 9, 31, 65, 250, 4099):
+        for groups in (1, 30, 4096, 300000):
+            for fp32 in (0, 1):
+                assert 1 <= host.segment(groups, n, 4, slots, fp32) <= n
