@@ -31,7 +31,9 @@ namespace walk4 {
 
 using namespace walk;
 
-enum { K_HYBC = 0, K_W7, K_HYBN, K_SYMC, K_W5, K_SYM, K_OMP6, K_NND2 };
+// (K_W7C: K_W7 in FP32 on x lines with boundary closures, see Shape4)
+enum { K_HYBC = 0, K_W7, K_HYBN, K_SYMC, K_W5, K_SYM, K_OMP6, K_NND2, K_W7C };
+constexpr bool w7_kind(int k) { return k == K_W7 || k == K_W7C; }
 constexpr bool char_kind(int k) { return k == K_HYBC || k == K_SYMC; }
 constexpr bool flag_kind(int k) { return k == K_HYBC || k == K_HYBN; }
 
@@ -45,7 +47,11 @@ __device__ __forceinline__ R rv(const R *ring, int col, int sv, int Q) {
 // the ring, and five blocks of the y and z walks an SM.  In x the faces of
 // four rows share a warp (a row of 512 takes 65 passes of 8 a lane group, where
 // 32 of one row would take 17 of them four times over with a nearly empty last);
-// WENO7's shorter faces gain nothing from it and keep one row.
+// WENO7's shorter faces gain nothing from it and keep one row, except in FP32
+// on x lines with closures, whose quotients hold up the whole pass that one
+// of a line's ends is in: two or three passes of each row, or one in eight of
+// four rows.  x sweep of 64^3 between walls 77 -> 50 us; one step of 64^3 with
+// closures on all faces 605 -> 444 us, of 128^3 2.76 -> 2.36 ms.
 template <int DIR, int KIND> struct Shape4 {
     static constexpr int LC = DIR == 0 ? (KIND == K_W7 ? 1 : 4) : 8, RING = DIR == 0 ? (KIND == K_W7 ? 64 : 16) : 12;
 };
@@ -186,19 +192,19 @@ __device__ __forceinline__ void face4(const Params &p, int dir, const R *ring, i
                                       int hflag, long long o0, long long sd, bool lo, bool hi,
                                       R *fb) {
     const bool near = (lo && F <= 3) || (hi && F >= n - 5);
-    if constexpr (!char_kind(KIND) && KIND != K_W7) {
+    if constexpr (!char_kind(KIND) && !w7_kind(KIND)) {
         constexpr int KA0 = KIND == K_W5 || KIND == K_NND2 ? 2 : 3, KB0 = KA0 == 2 ? 2 : 4;     // extents()
         constexpr int KA1 = KB0, KB1 = KA0;
         comp_sign<KIND, 0, RING, LC>(p, ring, col, F, near ? closure_class(0, lo, hi, KA0, KB0, F, n) : 0, hflag, fb);
         comp_sign<KIND, 1, RING, LC>(p, ring, col, F, near ? closure_class(1, lo, hi, KA1, KB1, F, n) : 0, hflag, fb);
         return;
     } else {
-    if (near && (KIND == K_W7 || (KIND == K_HYBC && hflag == 1))) {
-        if (KIND == K_W7) comp_face_closure<RING, LC, true>(ring, col, F, n, lo, hi, 3, 3, 3, 3, fb);
+    if (near && (w7_kind(KIND) || (KIND == K_HYBC && hflag == 1))) {
+        if (w7_kind(KIND)) comp_face_closure<RING, LC, true>(ring, col, F, n, lo, hi, 3, 3, 3, 3, fb);
         else              comp_face_closure<RING, LC, false>(ring, col, F, n, lo, hi, 3, 4, 4, 3, fb);
         return;
     }
-    if (KIND == K_W7) { face_w7<RING, LC>(ring, col, F, fb); return; }
+    if (w7_kind(KIND)) { face_w7<RING, LC>(ring, col, F, fb); return; }
     if (KIND == K_HYBC && hflag == 1) {
         R out[10];
         face_up7<RING, LC>(ring, col, F, out);
@@ -568,6 +574,8 @@ cudaError_t dir4k(const Params &p, int dir, cudaStream_t st) {
 template <bool UNI, bool EPS0, typename R>
 cudaError_t dir4(const Params &p, int dir, cudaStream_t st) {
     if (p.scheme_invis == 310 && p.charteric) return dir4k<UNI, EPS0, K_HYBC, R>(p, dir, st);
+    if constexpr (sizeof(R) == 4)
+        if (dir == 0 && (p.bnd_lo[0] || p.bnd_hi[0])) return launch_dir4<0, UNI, EPS0, K_W7C, 5, false, R>(p, st);
     return dir4k<UNI, EPS0, K_W7, R>(p, dir, st);
 }
 

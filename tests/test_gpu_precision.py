@@ -103,3 +103,22 @@ def test_fp32_form_tracks_fp64_on_the_ramp(maker, gpu_lib):
     assert np.all(pb[1][:, 0, :] == 0.0) and np.all(pb[3][:, 0, :] == 0.0)
     if case.cfg.bc_rpara[0] > 0:
         assert np.allclose(pb[4][:, 0, :], case.cfg.bc_rpara[0], rtol=1e-14)
+
+
+@pytest.mark.parametrize("dims", [(8, 9, 33), (41, 8, 10), (33, 67, 13), (70, 9, 9)])
+@pytest.mark.parametrize("dif_bound", [(1,) * 6, (1, 0, 0, 0, 0, 0), (0, 1, 0, 0, 0, 0)])
+def test_fp32_weno7_closed_x_lines(dims, dif_bound, gpu_lib):
+    """WENO7 in FP32 on x lines with closures at both ends or one: four rows a
+    warp, rows left over, lines shorter than a pass and a cell longer than
+    some; a uniform grid (a closed periodic direction) as well.  Against FP64
+    within the form's bound."""
+    for periodic in ((0, 0, 0), (1, 1, 1)):
+        case = cases.random_smooth_case(*dims, seed=31, dt=1e-3, iperiodic=periodic, dif_bound=dif_bound)
+        a = lib.Solver(case.cfg, case.prims, case.metrics)
+        a.set_sweep_impl(5)
+        b = lib.Solver(case.cfg, case.prims, case.metrics)
+        b.set_precision(1)
+        a.step(2)
+        b.step(2)
+        err = rel_l2(b.conserved(), a.conserved())
+        assert np.all(np.isfinite(err)) and np.all(err > 0) and np.all(err <= TOL_FP32_10STEPS), (periodic, err)
