@@ -36,6 +36,7 @@ namespace {
 using namespace walk;
 
 constexpr int RW = 4;          // warps per block
+template <typename R> constexpr int row_blocks() { return sizeof(R) == 8 ? 4 : 6; }     // blocks per SM
 
 template <typename R> struct Vec;
 template <> struct Vec<double> { using T = double2; static constexpr int N = 2; };
@@ -99,7 +100,7 @@ __device__ __forceinline__ void store4(float *f, const float (&v)[4]) {
 }
 
 template <bool UNI, bool EPS0, typename R, int LPR>
-__global__ void __launch_bounds__(32 * RW, sizeof(R) == 8 ? 4 : 6) k_row(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(32 * RW, row_blocks<R>()) k_row(const __grid_constant__ Params p, int seg_len) {
     using T = RowTile<R, LPR>;
     constexpr int N4 = 4 / Vec<R>::N, HALF = T::UNITS / 2;     // units of four points
     extern __shared__ __align__(16) unsigned char smem_row[];
@@ -126,11 +127,12 @@ __global__ void __launch_bounds__(32 * RW, sizeof(R) == 8 ? 4 : 6) k_row(const _
     auto split = [&](long long o, R d, R u, R v, R w, R Tt, R (&fp)[5], R (&fm)[5]) {
         split_point<0, UNI, EPS0>(p, o, d, u, v, w, Tt, fp, fm);
     };
-    // points -4 .. 3 of each row, one a lane
+    const int xs = (int)blockIdx.y * seg_len, xe = xs + seg_len < n ? xs + seg_len : n;     // this segment's cells
+    // points xs-4 .. xs+3 of each row, one a lane
     if (lane < 8 * T::ROWS) {
         const int rr = lane >> 3, t = lane & 7;
         const long long row2 = r0 + rr < nrows ? r0 + rr : nrows - 1;
-        const long long o = row_base(row2) + t - 4;
+        const long long o = row_base(row2) + xs + t - 4;
         R q5[5], fp[5], fm[5];
         load5(p, o, q5);
         split(o, q5[0], q5[1], q5[2], q5[3], q5[4], fp, fm);
@@ -140,7 +142,7 @@ __global__ void __launch_bounds__(32 * RW, sizeof(R) == 8 ? 4 : 6) k_row(const _
             reinterpret_cast<R *>(&tile.u[5 + m][rr][T::at(t / Vec<R>::N)])[t % Vec<R>::N] = fm[m];
         }
     }
-    for (int x0 = 0; x0 < n; x0 += T::C) {
+    for (int x0 = xs; x0 < xe; x0 += T::C) {
         const int i0 = x0 + 4 * il;                            // the lane's cells i0 .. i0+3
         // flags of the faces i0-1/2 .. i0+7/2
         int hf[5];
@@ -232,7 +234,7 @@ __global__ void __launch_bounds__(32 * RW, sizeof(R) == 8 ? 4 : 6) k_row(const _
                 }
             }
         }
-        if (x0 + T::C < n) {       // points x0+C-4 .. x0+C+3 open the next pass
+        if (x0 + T::C < xe) {      // points x0+C-4 .. x0+C+3 open the next pass
             __syncwarp();
             constexpr int NU = 8 / Vec<R>::N, M = 10 * T::ROWS * NU;
 #pragma unroll
@@ -263,17 +265,23 @@ cudaError_t prepare_r() {
 template <bool UNI, bool EPS0, typename R, int LPR>
 cudaError_t launch_lpr(const Params &p, cudaStream_t st) {
     const long long warps = ((long long)p.ny * p.nz + 32 / LPR - 1) / (32 / LPR);
-    k_row<UNI, EPS0, R, LPR><<<(unsigned)((warps + RW - 1) / RW), 32 * RW, RW * sizeof(RowTile<R, LPR>), st>>>(p);
+    // (segments of whole passes where the chip has slots left: a 500x12x12 UP7
+    // step on metric fields takes 151 us where the rows' four passes took 215)
+    const long long slots = 148LL * row_blocks<R>() * RW;
+    const int passes = (p.nx + 4 * LPR - 1) / (4 * LPR), fit = (int)(warps < slots ? slots / warps : 1);
+    const int len = fit >= passes ? 1 : (passes + fit - 1) / fit;              // passes a segment
+    const dim3 grid((unsigned)((warps + RW - 1) / RW), (unsigned)((passes + len - 1) / len));
+    k_row<UNI, EPS0, R, LPR><<<grid, 32 * RW, RW * sizeof(RowTile<R, LPR>), st>>>(p, len * 4 * LPR);
     return cudaGetLastError();
 }
 
-// lanes a row: the most that waste the fewest cells of a row's last pass
 template <bool UNI, bool EPS0, typename R>
 cudaError_t launch_r(const Params &p, cudaStream_t st) {
-    auto cells = [&](int lpr) { return (p.nx + 4 * lpr - 1) / (4 * lpr) * (4 * lpr); };
-    if (cells(32) <= cells(16) && cells(32) <= cells(8)) return launch_lpr<UNI, EPS0, R, 32>(p, st);
-    if (cells(16) <= cells(8)) return launch_lpr<UNI, EPS0, R, 16>(p, st);
-    return launch_lpr<UNI, EPS0, R, 8>(p, st);
+    switch (row_lanes(p.nx, (long long)p.ny * p.nz, 148LL * row_blocks<R>() * RW)) {
+    case 32: return launch_lpr<UNI, EPS0, R, 32>(p, st);
+    case 16: return launch_lpr<UNI, EPS0, R, 16>(p, st);
+    default: return launch_lpr<UNI, EPS0, R, 8>(p, st);
+    }
 }
 
 template <typename R>

@@ -229,6 +229,26 @@ inline bool march_is_faster(int nx, long long cells, bool uniform, bool fp32) {
 
 template <typename R> constexpr int segment_tail() { return sizeof(R) == 8 ? 0 : 2; }
 
+// Lanes a row of the UP7 x walk (ocfd_row.cu: 32, 16 or 8, four cells each): the
+// least time of a row's passes, each the work of all warps and the latency of
+// one, 0.46 of a full round of the chip's slots (0.45: 160x33x65 takes 16 lanes,
+// 297 us a step for 282; 0.48: 96^3 takes 32).  On large grids that is the choice
+// that wastes the fewest cells of a row's last pass, on small ones, which no
+// choice fills the chip with, a short chain of passes.  UP7 steps of FP64 against
+// the fewest wasted cells alone, us: 93x44x19 124 / 151, 130x40x40 218 / 269,
+// 160x33x65 282 / 335, 65x64x64 260 / 280, 200x100x100 1223 / 1280.
+inline int row_lanes(int nx, long long rows, long long slots) {
+    int best = 0;
+    long long least = 0;
+    for (int lanes = 32; lanes >= 8; lanes /= 2) {
+        const int per = 32 / lanes;
+        const long long warps = (rows + per - 1) / per, passes = (nx + 4 * lanes - 1) / (4 * lanes);
+        const long long t = passes * (100 * warps + 46 * slots);
+        if (!best || t < least) { best = lanes; least = t; }
+    }
+    return best;
+}
+
 template <int DIR> struct Shape;
 template <> struct Shape<0> { static constexpr int LC = 1, RING = 64; };
 template <> struct Shape<1> { static constexpr int LC = 8, RING = 16; };

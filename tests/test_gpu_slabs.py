@@ -124,6 +124,11 @@ def _distinct_case(name, world):
             for z0, _ in slabs.part_z(n * world, world)[1:]:
                 c.prims[4][z0 - 1] *= 3.0
         return c, ((lambda s: s.set_precision(1)) if "fp32" in name else None)
+    if name == "up7_walks":
+        # marches and 8 lanes a row on the whole grid, the ring and 32 on a slab
+        return cases.random_smooth_case(96, 50, 62 * world, seed=6, scheme_invis="UP7", curvilinear=True), None
+    if name == "up7_segments":          # whole rows on the whole grid, three segments of a row on a slab
+        return cases.random_smooth_case(300, 20, 30 * world, seed=7, scheme_invis="UP7", curvilinear=True), None
     c = cases.random_smooth_case(n, n + 2, n * world, seed=5, curvilinear=True, shock=True)
     return c, None
 
@@ -147,7 +152,7 @@ def _slab_flags(tmp_path, d, world):
 
 
 @pytest.mark.parametrize("name,world", [("tgv_weno7", 2), ("iso_hybrid", 3), ("iso_hybrid_fp32", 2),
-                                        ("curvilinear", 3)])
+                                        ("curvilinear", 3), ("up7_walks", 3), ("up7_segments", 3)])
 def test_distinct_slabs_equal_single_gpu(name, world, gpu_lib, tmp_path):
     """2 or 3 slab processes on one GPU, each with its own z slab of an
     n x n x (n world) grid and its neighbours' ghost planes through host

@@ -21,6 +21,7 @@ using std::fma; using std::fabs; using std::sqrt; using std::fmin; using std::fm
 extern "C" int march(int nx, long long cells, int uniform, int fp32) {
     return ocfd::walk::march_is_faster(nx, cells, uniform, fp32);
 }
+extern "C" int lanes(int nx, long long rows, long long slots) { return ocfd::walk::row_lanes(nx, rows, slots); }
 extern "C" int segment(long long groups, int n, int LY, long long slots, int fp32) {
     using namespace ocfd::walk;
     return segment_cells(groups, n, LY, slots, 3, fp32 ? segment_tail<float>() : segment_tail<double>());
@@ -36,6 +37,7 @@ def host(tmp_path_factory):
                     "-o", str(d / "host.so")], check=True)
     h = ctypes.CDLL(str(d / "host.so"))
     h.segment.argtypes = [ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_int]
+    h.lanes.argtypes = [ctypes.c_int, ctypes.c_longlong, ctypes.c_longlong]
     h.march.argtypes = [ctypes.c_int, ctypes.c_longlong, ctypes.c_int, ctypes.c_int]
     return h
 
@@ -66,3 +68,13 @@ def test_segments_of_fp32_lines(host):
         for groups in (1, 30, 4096, 300000):
             for fp32 in (0, 1):
                 assert 1 <= host.segment(groups, n, 4, slots, fp32) <= n
+
+
+@pytest.mark.parametrize("nx,rows,lanes", [(93, 836, 32), (74, 1456, 32), (65, 4096, 32), (130, 1600, 32),
+                                           (160, 2145, 32), (80, 6400, 32), (96, 9216, 8), (64, 4096, 16), (60, 2000, 16),
+                                           (32, 1024, 8), (60, 6000, 16), (12, 90000, 8), (160, 25600, 8),
+                                           (256, 65536, 32)])
+def test_row_lanes(host, nx, rows, lanes):
+    """Lanes a row of the UP7 x walk in FP64 (four blocks an SM): short
+    chains of passes on small grids, the fewest wasted cells on large ones."""
+    assert host.lanes(nx, rows, 148 * 4 * 4) == lanes
