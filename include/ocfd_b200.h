@@ -102,7 +102,8 @@ int ocfd_b200_set_metrics(ocfd_b200_ctx *ctx, const double *metrics13);
 int ocfd_b200_set_metric_mode(ocfd_b200_ctx *ctx, int mode);
 int ocfd_b200_uniform_metrics(const ocfd_b200_ctx *ctx);
 /* Inviscid sweep kernel variant: 4 (default) no block barriers: each warp
- * walks its own lines (4 x rows, or 8 y or z lines) through a ring of split
+ * walks its own lines (4 x rows, one for WENO7 but on FP32 rows with
+ * closures, or 8 y or z lines) through a ring of split
  * values in shared memory and forms every face, closure and line-end rule
  * in the walk; UP7, and a hybrid direction whose sensor pass marked almost
  * every face UP7 (the choice is read back once per step, after the sensor),

@@ -626,7 +626,8 @@ static int apply_bc(ocfd_b200_ctx *ctx) {
 // The UP7 walk leaves the two cells beside every non-UP7 face, and the ~10
 // cells at each bounded end of a line, to a per-cell fix-up kernel that
 // costs about as much as 80 cells of the walk; above a small fraction of
-// such cells the walk that forms every face in line is faster.
+// such cells the walk that forms every face in line is faster.  (The line was
+// fitted to earlier forms of both walks, on 256^3.)
 static bool walk4_wanted(const ocfd_b200_ctx *ctx, int d, unsigned nonup7) {
     const Params &p = ctx->p;
     // flag entries the count covers (with the grid split in z, the counts are

@@ -1,9 +1,11 @@
 // ocfd_device.cuh -- device-side arithmetic of the RHS path (sm_100a, FP64).
 //
-// Point formulas restate the reference scheme kernels; each keeps the
-// reference's expression order so nvcc contracts them the same way it does
-// the reference build (both use the default -fmad=true).  References are to
-// the OpenCFD-SCU tree.
+// Point formulas restate the reference scheme kernels: the split, the sensor
+// and the eigen-rows in the reference's expression order, the reconstructions
+// and the viscous differences in differences of their points with the
+// multiply-adds spelled out (fewer operations, less cancellation; they agree
+// with the reference's sums to rounding).  References are to the OpenCFD-SCU
+// tree.
 #pragma once
 #include <cstdint>
 
@@ -64,9 +66,9 @@ struct Params {
     double inv_h[3], inv_Ama;   // reciprocals for div_const
     double d0_h[3], d0_ih[3];   // divisor of the viscous scheme's difference (60 h or 840 h) and its reciprocal
     int sweep_impl;         // 4: the walks chosen per direction (default); 5: every face through the in-loop dispatch; 6: the in-line walk
-    // viscous divergence + RK of whole steps: 0 Ev tiles staged in shared
-    // memory in the precision form, read through L1/L2 in FP64 (each the
-    // faster there); 1 read through L1/L2; 2 staged
+    // viscous kernels of whole steps: 0 inputs staged in shared memory in the
+    // precision form on a million cells or more without closed faces, read
+    // through L1/L2 elsewhere (vis_staged); 1 read through L1/L2; 2 staged
     int vis_impl;
     // cells whose du the call-free sweep leaves to the fix-up kernel, per
     // direction (interior cell indices; capacity N each), and their counts
@@ -301,16 +303,6 @@ __device__ __forceinline__ double weno5_p(const double *s) { return weno5_core(s
 __device__ __forceinline__ double weno5_m(const double *s8) {
     const double v[6] = { s8[7], s8[6], s8[5], s8[4], s8[3], s8[2] };
     return weno5_core(v);
-}
-
-// UP7, src/OCFD_Schemes.cu:865-907
-__device__ __forceinline__ double up7_p(const double *s) {
-    return (-3.0*s[0] + 25.0*s[1] - 101.0*s[2] + 319.0*s[3] + 214.0*s[4]
-            - 38.0*s[5] + 4.0*s[6])/420.0;
-}
-__device__ __forceinline__ double up7_m(const double *s) {
-    return (-3.0*s[7] + 25.0*s[6] - 101.0*s[5] + 319.0*s[4] + 214.0*s[3]
-            - 38.0*s[2] + 4.0*s[1])/420.0;
 }
 
 // sign / minmod, src/OCFD_Schemes.cu:766-797 (minmod4 keeps the fmin of the

@@ -11,7 +11,10 @@
 #include "ocfd_fp32.cuh"
 #include "ocfd_tma.cuh"
 
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
+
+#include <mutex>
 
 namespace ocfd {
 
@@ -1132,6 +1135,43 @@ cudaError_t launch_vis_ev(const Params &p, int images, cudaStream_t st) {
         if (done) return e;
     }
     return p.mixed ? launch_vis_ev_t<float>(p, images, st) : launch_vis_ev_t<double>(p, images, st);
+}
+
+static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
+    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void *ptr = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &ptr, 12000, cudaEnableDefault, &q) ==
+                cudaSuccess && q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(ptr);
+        else
+            cudaGetLastError();
+    });
+    return fn;
+}
+
+// A 4-D tiled tensor map (FP64 or FP32 elements, no swizzle, out-of-range
+// elements read as zero): dims[0] innermost, strides in bytes of dims 1..3,
+// box in elements.  Returns false when the driver entry point is missing or
+// the layout breaks the copy engine's rules (16-byte aligned base and
+// strides, inner box a multiple of 16 bytes).
+static bool encode_map_4d(const void *base, int elem_bytes, const unsigned long long dims[4],
+                   const unsigned long long strides[3], const unsigned box[4], CUtensorMap *out) {
+    PFN_cuTensorMapEncodeTiled_v12000 fn = encode_fn();
+    if (!fn || !base || ((unsigned long long)base & 15)) return false;
+    for (int i = 0; i < 3; i++)
+        if (strides[i] % 16) return false;
+    if (((unsigned long long)box[0] * elem_bytes) % 16) return false;
+    cuuint64_t d[4] = { dims[0], dims[1], dims[2], dims[3] };
+    cuuint64_t st[3] = { strides[0], strides[1], strides[2] };
+    cuuint32_t bx[4] = { box[0], box[1], box[2], box[3] };
+    cuuint32_t estr[4] = { 1, 1, 1, 1 };
+    CUresult r = fn(out, elem_bytes == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
+                    const_cast<void *>(base), d, st, bx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS;
 }
 
 // persistent grid of the staged viscous kernels: blocks per SM from their

@@ -1,5 +1,5 @@
 // ocfd_march.cu -- the UP7 walk of the y and z sweeps as per-lane marches
-// (sm_100a; FP64, and FP32 for the precision form), and the tensor-map encoder.
+// (sm_100a; FP64, and FP32 for the precision form).
 //
 // Same results as the UP7 walk of ocfd_sweep3.cu (the reference's
 // OCFD_d{y,z}1/2 chain with the hybrid scheme's UP7 faces, src/OCFD_Schemes.cu:159-381,
@@ -31,9 +31,7 @@
 #include "ocfd_tma.cuh"
 #include "ocfd_walk.cuh"
 
-#include <cudaTypedefs.h>
-
-#include <mutex>
+#include <cuda_runtime.h>
 
 namespace ocfd {
 
@@ -262,38 +260,6 @@ cudaError_t march_prepare() {
     one(set_smem<1, true, false, float>());  one(set_smem<2, true, false, float>());
     one(set_smem<1, false, false, float>()); one(set_smem<2, false, false, float>());
     return e;
-}
-
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *ptr = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &ptr, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess && q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(ptr);
-        else
-            cudaGetLastError();
-    });
-    return fn;
-}
-
-bool encode_map_4d(const void *base, int elem_bytes, const unsigned long long dims[4],
-                   const unsigned long long strides[3], const unsigned box[4], CUtensorMap *out) {
-    PFN_cuTensorMapEncodeTiled_v12000 fn = encode_fn();
-    if (!fn || !base || ((unsigned long long)base & 15)) return false;
-    for (int i = 0; i < 3; i++)
-        if (strides[i] % 16) return false;
-    if (((unsigned long long)box[0] * elem_bytes) % 16) return false;
-    cuuint64_t d[4] = { dims[0], dims[1], dims[2], dims[3] };
-    cuuint64_t st[3] = { strides[0], strides[1], strides[2] };
-    cuuint32_t bx[4] = { box[0], box[1], box[2], box[3] };
-    cuuint32_t estr[4] = { 1, 1, 1, 1 };
-    CUresult r = fn(out, elem_bytes == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
-                    const_cast<void *>(base), d, st, bx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS;
 }
 
 // The march covers the UP7 walk's schemes (the hybrid scheme, UP7 without

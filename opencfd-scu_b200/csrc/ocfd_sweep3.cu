@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep3(const __grid_constant_
     // ring spans both windows
     constexpr bool SYNC2 = 2 * LY + 6 >= RING;
     static_assert(FAST || sizeof(R) == 8, "the in-loop dispatch is FP64 only");
+    static_assert(!FAST || DIR != 0, "the UP7 walk of x is k_row (ocfd_row.cu)");
     __shared__ R ring_all[SW][10 * RING * LC];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int col = lane % LC, ly = lane / LC;
@@ -116,8 +117,7 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep3(const __grid_constant_
             slow = !up7_face(p, hf) || near_closure(p, DIR, y0 - 1, n);
             if (!slow) face_up7_sum<RING, LC>(ring, col, y0 - 1, cur);
         } else {
-            if constexpr (sizeof(R) == 8 && !FAST)
-                face_flux<RING, LC, UNI>(p, DIR, ring, col, y0 - 1, n, hf, base + (long long)(y0 - 1) * sd, sd, cur);
+            face_flux<RING, LC, UNI>(p, DIR, ring, col, y0 - 1, n, hf, base + (long long)(y0 - 1) * sd, sd, cur);
         }
     }
 #pragma unroll
@@ -151,8 +151,7 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep3(const __grid_constant_
             slow = valid && (!up7_face(p, hflag) || near_closure(p, DIR, F, n));
             if (valid && !slow) face_up7_sum<RING, LC>(ring, col, F, cur);
         } else {
-            if constexpr (sizeof(R) == 8)
-                if (valid) face_flux<RING, LC, UNI>(p, DIR, ring, col, F, n, hflag, base + (long long)F * sd, sd, cur);
+            if (valid) face_flux<RING, LC, UNI>(p, DIR, ring, col, F, n, hflag, base + (long long)F * sd, sd, cur);
         }
         R prv[NV];
 #pragma unroll
@@ -185,8 +184,7 @@ __global__ void __launch_bounds__(32 * SW, MINB) k_sweep3(const __grid_constant_
             if constexpr (FAST) {
                 const R cf = up7_scale(aj, p.inv_h[DIR]);
 #pragma unroll
-                for (int m = 0; m < 5; m++)
-                    du[m * N + ci] = DIR == 0 ? cf * (cur[m] - prv[m]) : fma_r(cf, cur[m] - prv[m], old[m]);
+                for (int m = 0; m < 5; m++) du[m * N + ci] = fma_r(cf, cur[m] - prv[m], old[m]);
             } else {
                 if (DIR == 0) add_du<true>(du, N, ci, aj, h, ih, cur, prv, old);
                 else          add_du<false>(du, N, ci, aj, h, ih, cur, prv, old);

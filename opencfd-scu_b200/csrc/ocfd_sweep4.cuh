@@ -282,9 +282,7 @@ __device__ __forceinline__ void du_rule_cell(const Params &p, const R *ring, int
     }
 }
 
-// MINB: resident blocks per SM the register budget is fitted to; 3 (168
-// registers, a few spills) runs faster than 2 (no spills) on the
-// characteristic faces.
+// MINB: resident blocks per SM the register budget is fitted to (dir4s).
 // The walk: a warp covers LC lines and LY = 32 / LC consecutive faces of
 // each per pass, from the one left of the segment's first cell on.  Per pass
 // every lane splits one new point into the ring, forms its face's flux into

@@ -1,5 +1,5 @@
 // ocfd_tma.cuh -- bulk tensor copies into shared memory (sm_100a): mbarrier
-// helpers, the 4-D tile load and the host-side tensor-map encoder.  Every
+// helpers and the 4-D tile load (the tensor maps: ocfd_kernels.cu).  Every
 // tensor map here covers this GPU's own memory, and no load multicasts
 // across a cluster.
 #pragma once
@@ -57,13 +57,5 @@ __device__ __forceinline__ void prefetch_l1(const void *ptr) {
 }
 
 }  // namespace tma
-
-// A 4-D tiled tensor map (FP64 or FP32 elements, no swizzle, out-of-range
-// elements read as zero): dims[0] innermost, strides in bytes of dims 1..3,
-// box in elements.  Returns false when the driver entry point is missing or
-// the layout breaks the copy engine's rules (16-byte aligned base and
-// strides, inner box a multiple of 16 bytes).
-bool encode_map_4d(const void *base, int elem_bytes, const unsigned long long dims[4],
-                   const unsigned long long strides[3], const unsigned box[4], CUtensorMap *out);
 
 }  // namespace ocfd
