@@ -429,22 +429,22 @@ SWITCH_MODEL = os.path.join(os.path.dirname(os.path.abspath(__file__)), "opencfd
                             "switch_c1c3.npz")
 
 # Measured DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per cell
-# for one stage's launches of each family, from one ncu capture of the same
-# kernels at 160^3 (profiles/stage_traffic_iso160.txt); the traffic scales with
+# for one stage's launches of each family, from one ncu capture of these
+# kernels at 160^3 (profiles/stage_counters.txt); the traffic scales with
 # the cells processed, so the bench line reports it times the cells of a launch.
 TRAFFIC_PER_CELL = {
-    "inviscid_sweeps": 304.6,       # 3 sweeps + 3 fix-ups
-    "viscous_rk_update": 385.6,     # k_vis_ev + k_vis_div (Ev ghost fill not captured)
+    "inviscid_sweeps": 308.8,       # 3 sweeps + 3 fix-ups
+    "viscous_rk_update": 387.3,     # k_vis_ev + k_vis_div
 }
-TRAFFIC_SOURCE = "ncu capture at 160^3 scaled by cells (profiles/stage_traffic_iso160.txt)"
+TRAFFIC_SOURCE = "ncu capture at 160^3 scaled by cells (profiles/stage_counters.txt)"
 
 # FP64 operations executed per cell and stage (2 x DFMA + DADD + DMUL, counted
-# by ncu over one stage's kernels: profiles/fp64_flops_iso160_tgv128_ramp256.txt);
+# by ncu over one stage's kernels: profiles/stage_counters.txt);
 # times the measured rate, the FP64 rate the whole stage sustains.  The hybrid
 # count depends on how many faces the sensor flags (isotropic turbulence: UP7
 # almost everywhere).
-FP64_FLOP_PER_CELL_STAGE = {"iso": 2353.0, "tgv": 7353.0, "ramp": 10712.0}
-FLOP_SOURCE = "ncu executed FP64 instructions per stage (profiles/fp64_flops_iso160_tgv128_ramp256.txt)"
+FP64_FLOP_PER_CELL_STAGE = {"iso": 1622.0, "tgv": 5341.0, "ramp": 8987.0}
+FLOP_SOURCE = "ncu executed FP64 instructions per stage (profiles/stage_counters.txt)"
 
 
 def run_reference(args, rank, world):

@@ -1076,6 +1076,9 @@ cudaError_t launch_ghost32(const Params &p, float *const *fields, const int *dir
 
 
 
+// (With closures the metric fields are read: constant metrics are kept for grids
+// periodic in all three directions, detect_uniform, and closures in a periodic
+// direction are rare.)
 template <typename R>
 static cudaError_t launch_vis_ev_t(const Params &p, int images, cudaStream_t st) {
     const dim3 nb((unsigned)(((p.nx + VT_X - 1) / VT_X) * ((p.ny + VT_Y - 1) / VT_Y)), (unsigned)p.nz);

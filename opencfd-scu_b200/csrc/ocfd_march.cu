@@ -18,8 +18,8 @@
 // Primitives, the cell's du and (curvilinear grids) the metrics are copied
 // to the lane's own shared-memory slots by cp.async STAGES - 1 points ahead; a
 // lane reads only what it copied, so the walk takes no barrier at all.
-// Bounds: FP64 by memory latency and bandwidth (120 B a cell and direction,
-// 53 % of DRAM peak with 12 warps an SM), FP32 by instruction issue (68 %).
+// Bounds at 160^3: FP64 by memory latency and bandwidth (120 B a cell and direction,
+// 51 to 55 % of DRAM peak with 12 warps an SM), FP32 by instruction issue (70 %).
 // At 160^3, y / z: FP64 110 / 108 us against 158 / 171 for the ring walk; FP32
 // 78 / 79 us against 112 / 107 for a march over tiles from the tensor copy
 // engine with a register window of split values.

@@ -18,8 +18,8 @@
 // nothing is passed between lanes.  16-byte units of FP64 are kept even ones
 // first, then odd ones, so that the lanes of a read touch consecutive units.
 // The last eight points of a pass are the first eight of the next.
-// Bound by the shared-memory pipe (68 % of its wavefronts in FP64) and FP32
-// issue (72 %).  At 160^3: 100 us in FP64 against 139 for the one-cell-a-lane
+// Bound in FP64 by the FP64 pipe and the shared-memory one between them (45 and
+// 44 % of peak at 160^3, a quarter of the warps an SM holds), in FP32 by issue (72 %).  At 160^3: 100 us in FP64 against 139 for the one-cell-a-lane
 // ring.  With the marches, the sweeps of a 256^3 stage: 1.27 against 1.39 ms
 // (FP64), 0.75 against 0.83 (FP32).
 #include "ocfd_walk.cuh"
